@@ -1,0 +1,25 @@
+// cand.h -- host interface of the candidate pass.
+#pragma once
+#include "ts_host.h"
+
+namespace tsb {
+
+constexpr int kCandSlice = 4096;             // vertices per CTA the cluster size aims at
+constexpr size_t kCandSmem = 220 * 1024;     // dynamic shared memory a CTA may ask for
+
+struct CandPlan {
+  int cs = 0;               // CTAs of the cluster; 0: the state does not fit
+  int32_t rpc = 0, cpc = 0; // rows and columns per CTA (multiples of 4)
+  int32_t fav = 0;          // every c*w >= 0
+  int64_t plus = 0;         // upper bound of c*w
+  size_t smem = 0;
+};
+// Slices for a given cluster size within `limit` bytes of shared memory.
+CandPlan cand_slices(const ts_graph* g, int32_t problem, int32_t m, bool wide, int cs, size_t limit);
+// The plain form's choice of cluster size.
+CandPlan cand_plan(const ts_graph* g, int32_t problem, int32_t m, bool wide);
+// `solver` points to a DevSolver<KeyT> (KeyT by `wide`).
+cudaError_t launch_cand(int32_t problem, int kind, bool wide, const DevGraph& g, const void* solver, int cs, size_t smem,
+                        cudaStream_t st, long long budget);
+
+}  // namespace tsb

@@ -18,6 +18,7 @@
 #include <unordered_set>
 #include <vector>
 
+#include "cand.h"
 #include "sweep.cuh"
 #include "ts_host.h"
 
@@ -410,6 +411,8 @@ struct ts_solver {
   bool external_draws = false;  // perturbation events given by the caller (no more are drawn)
   bool initialized = false;
   int64_t admitted_target = 0;
+  CandPlan cand;          // candidate pass (TS_PASS_AUTO); cs 0: sweeps only
+  int64_t backoff = 1;    // sweeps to run after the next hand-over (finish_batch)
   DevState* h_st = nullptr;  // pinned mirror
 
   template <class KeyT>
@@ -434,6 +437,7 @@ struct ts_solver {
     s.fast_ecap = fast_ecap;
     s.n_slices = n_slices;
     s.w16 = w16;
+    s.cand_rpc = cand.rpc; s.cand_cpc = cand.cpc; s.cand_fav = cand.fav; s.cand_plus = cand.plus;
     s.P = P;
     s.sol_in = sol_in.as<int32_t>(); s.sol_out = sol_out.as<int32_t>();
     s.vg_in = vg_in.as<KeyT>(); s.vg_out = vg_out.as<KeyT>();
@@ -467,9 +471,12 @@ ts_status write_state(ts_solver* s) {
   return TS_OK;
 }
 
+// `count` sweep launches; guard: each runs only while a candidate launch left
+// iterations to it (DevState::owed).
 template <class KeyT>
-ts_status launch_batch(ts_solver* s, int count) {
+ts_status launch_batch(ts_solver* s, int count, bool guard) {
   DevSolver<KeyT> d = s->dev<KeyT>();
+  d.guard = guard ? 1 : 0;
   DevGraph g = s->g->dev();
   cudaError_t e = s->p.problem == P_MDP
                       ? launch_iter_st<P_MDP, KeyT>(s->g->kind, g, d, s->grid, s->dyn_smem, s->g->stream, count)
@@ -675,6 +682,7 @@ ts_status ts_solver_create(ts_graph* g, const ts_params* p, ts_solver** out) {
   s->grid = s->n_row_blocks * s->n_chunks * s->n_slices;
   s->stage_bytes = tg.stage_bytes;
   s->dyn_smem = tg.smem;
+  if (p->pass == TS_PASS_AUTO) s->cand = cand_plan(g, p->problem, m, s->wide);
   const int32_t g_eff = std::min(p->gamma, n);
   s->num_pert = std::max(1, g_eff / 2);  // GPU-MAXBS-CSR.cu:433-434
   int64_t pert_moves = p->problem == TS_PROBLEM_MAXBS ? (p->max_iter / p->piter + 1) * s->num_pert : 0;
@@ -781,6 +789,7 @@ ts_status prepare_batch(ts_solver* s, int64_t k, int64_t* admitted) {
     sub = std::min<int64_t>(sub, (s->window_events - 2) * (int64_t)s->p.piter);
   }
   s->h_st->target = s->h_st->iter + sub;
+  s->h_st->owed = 0;
   ts_status rc;
   if ((rc = prepare_draws(s, sub)) != TS_OK) return rc;
   if ((rc = write_state(s)) != TS_OK) return rc;
@@ -789,19 +798,41 @@ ts_status prepare_batch(ts_solver* s, int64_t k, int64_t* admitted) {
   return TS_OK;
 }
 
-ts_status enqueue_launches(ts_solver* s, int64_t launches) {
+ts_status enqueue_sweeps(ts_solver* s, int64_t launches, bool guard) {
   while (launches > 0) {
     int c = (int)std::min<int64_t>(launches, 1 << 20);
-    ts_status rc = s->wide ? launch_batch<long long>(s, c) : launch_batch<int32_t>(s, c);
+    ts_status rc = s->wide ? launch_batch<long long>(s, c, guard) : launch_batch<int32_t>(s, c, guard);
     if (rc != TS_OK) return rc;
     launches -= c;
   }
   return TS_OK;
 }
 
+// Iterations of one candidate launch: up to about a second.
+constexpr int64_t kCandLaunchIters = 1 << 16;
+
+// `iters` iterations: candidate launches, and one sweep launch that runs
+// only if the candidate pass stopped at an iteration it leaves to a sweep.
+// What is still missing then is topped up by finish_batch.
+ts_status enqueue_launches(ts_solver* s, int64_t iters) {
+  if (iters <= 0) return TS_OK;
+  if (!s->cand.cs) return enqueue_sweeps(s, iters, false);
+  const DevGraph g = s->g->dev();
+  const DevSolver<long long> d8 = s->dev<long long>();
+  const DevSolver<int32_t> d4 = s->dev<int32_t>();
+  const void* d = s->wide ? static_cast<const void*>(&d8) : &d4;
+  for (; iters > 0; iters -= kCandLaunchIters) {
+    const cudaError_t e = launch_cand(s->p.problem, s->g->kind, s->wide, g, d, s->cand.cs, s->cand.smem, s->g->stream,
+                                      std::min<int64_t>(iters, kCandLaunchIters));
+    if (e != cudaSuccess) return cuda_fail(e, "candidate kernel launch");
+  }
+  return enqueue_sweeps(s, 1, true);
+}
+
 // Waits for the admitted batch; tops it up when exact passes consumed launches.
 ts_status finish_batch(ts_solver* s) {
   ts_status rc;
+  int64_t last = s->h_st->iter;
   for (int guard = 0; guard < 1 << 20; guard++) {
     if ((rc = read_state(s)) != TS_OK) return rc;
     if (s->h_st->err) {
@@ -809,7 +840,18 @@ ts_status finish_batch(ts_solver* s) {
       return TS_ERR_DEVICE;
     }
     if (s->h_st->done || s->h_st->iter >= s->admitted_target) return TS_OK;
-    if ((rc = enqueue_launches(s, s->admitted_target - s->h_st->iter + 1)) != TS_OK) return rc;
+    const int64_t left = s->admitted_target - s->h_st->iter;
+    if (!s->cand.cs) {
+      if ((rc = enqueue_sweeps(s, left + 1, false)) != TS_OK) return rc;
+      continue;
+    }
+    // The candidate pass stopped: some sweeps, then it tries again.  Stops in
+    // quick succession (ties everywhere) double the sweeps between tries.
+    s->backoff = s->h_st->iter - last > 4 * s->backoff ? 1 : std::min<int64_t>(2 * s->backoff, 4096);
+    last = s->h_st->iter;
+    const int64_t sweeps = std::min<int64_t>(left, s->backoff);
+    if ((rc = enqueue_sweeps(s, sweeps, false)) != TS_OK) return rc;
+    if ((rc = enqueue_launches(s, left - sweeps)) != TS_OK) return rc;
   }
   set_error("no progress");
   return TS_ERR_DEVICE;

@@ -1305,7 +1305,7 @@ iter_kernel(const DevGraph g, const DevSolver<KeyT> s) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   DevState* st = s.st;
-  if (st->done || st->iter >= st->target) return;
+  if (st->done || st->iter >= st->target || (s.guard && st->owed <= 0)) return;
   const int mode = st->mode;
   const long long iter = st->iter;
   const long long D64 = st->best - st->cur;
@@ -1353,7 +1353,10 @@ iter_kernel(const DevGraph g, const DevSolver<KeyT> s) {
   }
   block_best(k, i, sh.red);
   decide_apply<PROB, ST, KeyT>(g, s, mode, k, i, sh);
-  if (threadIdx.x == 0) st->counter = 0;
+  if (threadIdx.x == 0) {
+    st->counter = 0;
+    if (s.guard) st->owed -= 1;
+  }
 }
 
 }  // namespace tsb

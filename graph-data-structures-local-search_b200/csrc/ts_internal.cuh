@@ -79,7 +79,7 @@ struct DevState {
   int32_t done;
   int32_t stopped;
   int32_t err;
-  int32_t pad;
+  int32_t owed;           // iterations a candidate launch left to guard launches of the sweeps
 };
 
 template <class KeyT>
@@ -107,6 +107,12 @@ struct DevSolver {
   // WSwap: 1 when the matrix holds 16-bit weights (every |w| <= 32767), read
   // through W as int16_t; 0: 32-bit.
   int32_t w16;
+  // Candidate pass (cand.cuh): CTAs' slices of rows and columns (0: off),
+  // whether every c*w >= 0 (Max Bisection without negative weights) and the
+  // upper bound of c*w over the graph's edges.
+  int32_t cand_rpc, cand_cpc, cand_fav;
+  int32_t guard;          // this launch runs only while DevState::owed > 0
+  int64_t cand_plus;
   int64_t P;
   int32_t* sol_in;
   int32_t* sol_out;

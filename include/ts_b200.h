@@ -71,8 +71,12 @@ typedef enum ts_tenure { TS_TENURE_REF = 0, TS_TENURE_FIXED = 1 } ts_tenure;
  *   once for all 32 rows (32-bit keys only; 64-bit keys use TS_PASS_ROWS).
  * TS_PASS_ROWS: a few rows per tile, each pair looked up in its row's staged
  *   structure (fewer, cheaper tiles: small instances).
- * TS_PASS_AUTO: TILE from 2^22 swap pairs per iteration up (CSR with
- *   MDP or a negative weight: ROWS), else ROWS. */
+ * TS_PASS_AUTO: the candidate pass, which finds the same best pair from the
+ *   rows and columns whose bounds can reach it and runs its iterations in one
+ *   launch (about 290,000 vertices at most with 32-bit keys).  Iterations it
+ *   does not settle (ties everywhere, no allowed pair), and larger graphs:
+ *   TILE from 2^22 swap pairs per iteration up (CSR with MDP or a negative
+ *   weight: ROWS), else ROWS. */
 typedef enum ts_pass { TS_PASS_AUTO = 0, TS_PASS_TILE = 1, TS_PASS_ROWS = 2 } ts_pass;
 
 typedef struct ts_graph ts_graph;
@@ -89,7 +93,7 @@ typedef struct ts_graph_info {
   int64_t bitset_words_per_row;
 } ts_graph_info;
 
-/* Launch geometry of a solver's iteration kernel (no counterpart in the
+/* Launch geometry of a solver's sweep kernel (no counterpart in the
  * reference, whose kernels use one thread per pair): ts_solver_info. */
 typedef struct ts_solver_info {
   int32_t grid;           /* CTAs per iteration launch (one tile each) */
@@ -212,10 +216,11 @@ ts_status ts_solver_step(ts_solver* s, int64_t k, int64_t* done_iters);
  *   ts_solver_prepare(s, k, &adm)  synchronises, admits adm <= k iterations
  *       (bounded by max_iter; MaxBS also by its staged perturbation draws,
  *       about 62*piter per call) and stages what they need;
- *   ts_solver_enqueue(s, j)        puts j iteration launches on the solver's
- *       stream and returns at once; launches past the admitted target do nothing;
+ *   ts_solver_enqueue(s, j)        puts the launches of j iterations on the solver's
+ *       stream and returns at once; those past the admitted target do nothing;
  *   ts_solver_sync(s, &iter)       waits, completes the admitted iterations if
- *       exact re-evaluation passes consumed launches, checks the device error
+ *       exact re-evaluation passes or iterations that the candidate pass left
+ *       to a sweep consumed launches, checks the device error
  *       word; iter = iteration counter. */
 ts_status ts_solver_prepare(ts_solver* s, int64_t k, int64_t* prepared);
 ts_status ts_solver_enqueue(ts_solver* s, int64_t k);
