@@ -30,6 +30,7 @@
 #include <thread>
 #include <vector>
 
+#include "cand.h"
 #include "packed.cuh"
 #include "ts_host.h"
 
@@ -47,6 +48,8 @@ struct BatchJobDev {
   int32_t orig;             // index in the caller's job array
   int32_t adj_mask;         // CSR: adjacent pairs masked out of the w-free sweep
   int32_t tile_rows, fast, fast_ecap;  // tile shape (tile_geometry)
+  int32_t cand_rpc, cand_cpc, cand_fav;  // candidate pass (cand_persist); 0: tiles only
+  long long cand_plus, cand_pairs;
   const int32_t* init;      // MDP: m ids; MaxBS: part[n]
   const long long* draws;   // MaxBS perturbation events x num_pert
   long long draw_events;
@@ -81,6 +84,10 @@ __device__ DevSolver<KeyT> slot_solver(const BatchJobDev& J, const SlotPool<KeyT
   s.tile_rows = J.tile_rows;
   s.fast = J.fast;
   s.fast_ecap = J.fast_ecap;
+  s.n_slices = 1;
+  s.cand_rpc = J.cand_rpc; s.cand_cpc = J.cand_cpc; s.cand_fav = J.cand_fav;
+  s.cand_plus = J.cand_plus; s.cand_pairs = J.cand_pairs;
+  s.guard = 0;
   s.w16 = 0;  // slot pools hold 32-bit matrices
   s.P = (long long)s.m * s.delta;
   s.sol_in = P.sol_in + slot * P.s_m;
@@ -114,6 +121,7 @@ batch_kernel(const BatchJobDev* __restrict__ jobs, int njobs, BatchResultDev* __
   __shared__ TailShared sh;
   __shared__ int s_job;
   __shared__ CtaRec s_rec;
+  __shared__ CandShared<KeyT> s_cand;
   __shared__ long long sc[kMaxTPB / 32];
   __shared__ int32_t s_cnt[kMaxTPB];
   for (;;) {
@@ -130,7 +138,7 @@ batch_kernel(const BatchJobDev* __restrict__ jobs, int njobs, BatchResultDev* __
       __threadfence();
     }
     cl.sync();
-    cluster_iterate<PROB, ST, KeyT>(g, s, J.max_iter, cl, sh, s_rec);
+    cluster_iterate<PROB, ST, KeyT>(g, s, J.max_iter, cl, sh, s_rec, s_cand);
     if (rank == 0) slot_finish<PROB, KeyT>(g, s, out + J.orig, best_out + J.sol_off, sc);
   }
 }
@@ -261,8 +269,13 @@ ts_status plan_group(Group& G, std::vector<BatchJobDev>& table, int64_t budget_b
     J.chunk_cols = tg.chunk_cols;
     J.n_chunks = tg.n_chunks;
     J.stage_bytes = tg.stage_bytes;
-    const size_t need = tg.smem;
-    smem = std::max(smem, need);
+    const CandPlan cp = cand_persist(H.g, PROB, H.m, sizeof(KeyT) == 8, H.p.pass, cs);
+    J.cand_rpc = cp.cs ? cp.rpc : 0;
+    J.cand_cpc = cp.cpc;
+    J.cand_fav = cp.fav;
+    J.cand_plus = cp.plus;
+    J.cand_pairs = cp.pairs;
+    smem = std::max(smem, std::max(tg.smem, cp.cs ? cp.smem : (size_t)0));
     max_m = std::max<long long>(max_m, H.m);
     max_n = std::max<long long>(max_n, H.n);
     max_ldc = std::max<long long>(max_ldc, ldc);
@@ -472,7 +485,7 @@ ts_status ts_batch_create(const ts_batch_job* jobs, int32_t count, const ts_batc
   double total = 0;
   for (auto& H : hj) total += H.work;
   for (auto& H : hj) {
-    const int32_t cs = H.cluster ? H.cluster : auto_cluster(H.work, total, sms);
+    const int32_t cs = H.cluster ? H.cluster : (H.p.pass == TS_PASS_AUTO ? cand_cluster(H.n) : auto_cluster(H.work, total, sms));
     Group* G = nullptr;
     for (auto& x : b->groups)
       if (x.problem == H.p.problem && x.kind == H.kind && x.wide == H.wide && x.cluster == cs) G = &x;

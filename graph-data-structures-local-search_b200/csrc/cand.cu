@@ -102,8 +102,26 @@ CandPlan cand_slices(const ts_graph* g, int32_t problem, int32_t m, bool wide, i
   p.cpc = ((delta + cs - 1) / cs + 3) & ~3;
   p.smem = cand_layout(g->n, p.rpc, p.cpc, wide ? 8 : 4, p.plus > 0).total;
   if (p.smem <= limit) p.cs = cs;
+  // Looking up 64 pairs a thread takes about as long as a small sweep launch.
+  p.pairs = 64 * kCandTPB;
   return p;
 }
+
+CandPlan cand_persist(const ts_graph* g, int32_t problem, int32_t m, bool wide, int32_t pass, int cs) {
+  if (pass != TS_PASS_AUTO) return CandPlan{};
+  CandPlan p = cand_slices(g, problem, m, wide, cs, kCandPersistSmem);
+  if (!p.cs) return CandPlan{};
+  // The cluster's own sweep is the alternative: it passes eight pairs or more
+  // in the time of one candidate lookup.
+  p.pairs = std::max<int64_t>(64 * 256, (int64_t)m * (g->n - m) / 8 / cs);
+  return p;
+}
+
+// One CTA while the batch has solves for every SM: per iteration one 256-thread
+// CTA against two took 4.5 against 4.2 us (MDP, n = 5,000) and 33 against 21 us
+// (Max Bisection, n = 3,000) -- less than twice as fast on twice the SMs.
+// Larger solves need the second CTA's shared memory.
+int cand_cluster(int32_t n) { return n <= 6144 ? 1 : (n <= 16384 ? 2 : 4); }
 
 CandPlan cand_plan(const ts_graph* g, int32_t problem, int32_t m, bool wide) {
   // A CTA scans about 4,000 positions in the time of one cluster barrier;

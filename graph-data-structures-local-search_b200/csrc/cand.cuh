@@ -44,7 +44,6 @@ constexpr int kCandTPB = 512;        // threads per CTA of the plain form
 constexpr int kCandMaxCluster = 16;
 constexpr int kCandList = 2048;      // candidates a CTA can hold per side
 constexpr int kCandStage = 1024;     // candidate columns staged per round of N
-constexpr int kCandPairs = 64;       // N: pairs per thread beyond which the sweeps take over
 constexpr int kCandHeavy = 1024;     // E: rows of more entries are walked by the whole CTA
 constexpr int kCandHeavyList = 64;
 
@@ -53,6 +52,7 @@ enum { kCandEnd = 0, kCandBail = 1 };
 struct CandLayout {
   uint32_t va, vb, ta, tb, ua, ub, rl, cl, map, total;
   uint32_t map_bytes;
+  int32_t rcap, ccap;  // list lengths
 };
 // Shared memory of one CTA: rpc rows and cpc columns (multiples of 4), lists,
 // and one area that is the candidate-column bitmap (E) or the staged columns (N).
@@ -65,8 +65,10 @@ __host__ __device__ inline CandLayout cand_layout(int32_t n, int32_t rpc, int32_
   L.tb = off; off += 4u * cpc;
   L.ua = off; off += 4u * rpc;
   L.ub = off; off += 4u * cpc;
-  L.rl = off; off += 4u * kCandList;
-  L.cl = off; off += 4u * kCandList;
+  L.rcap = rpc < kCandList ? rpc : kCandList;
+  L.ccap = cpc < kCandList ? cpc : kCandList;
+  L.rl = off; off += 4u * (uint32_t)L.rcap;
+  L.cl = off; off += 4u * (uint32_t)L.ccap;
   L.map = off;
   L.map_bytes = edges ? 16u * (uint32_t)((n + 127) / 128) : 0u;
   const uint32_t stage = (uint32_t)(8 + kb) * kCandStage;
@@ -486,7 +488,7 @@ __device__ int cand_run(const DevGraph& g, const DevSolver<KeyT>& s, long long s
           const bool nt = ta[i] <= now;
           if ((nt && nt_ok && x + Bm + pl >= LB) || x + BA + pl >= LT) {
             const int32_t at = atomicAdd(&sh.nrow, 1);
-            if (at < kCandList) rl[at] = i;
+            if (at < L.rcap) rl[at] = i;
           }
         }
         for (int32_t j = tid; j < nc; j += T) {
@@ -494,7 +496,7 @@ __device__ int cand_run(const DevGraph& g, const DevSolver<KeyT>& s, long long s
           const bool nt = tb[j] <= now;
           if ((nt && nt_ok && x + Am + pl >= LB) || x + AA + pl >= LT) {
             const int32_t at = atomicAdd(&sh.ncol, 1);
-            if (at < kCandList) cll[at] = ids ? ub[j] : j;
+            if (at < L.ccap) cll[at] = ids ? ub[j] : j;
           }
         }
         cl.sync();
@@ -511,8 +513,8 @@ __device__ int cand_run(const DevGraph& g, const DevSolver<KeyT>& s, long long s
         if (tid == 0) sh.pre[0] = 0;
         const int32_t mr = __reduce_max_sync(0xffffffffu, cr), mc = __reduce_max_sync(0xffffffffu, cc);
         const int32_t tc = __shfl_sync(0xffffffffu, incl, 31);
-        if (mr > kCandList || mc > kCandList) bail = true;
-        if (!ids && (long long)mr * tc > (long long)kCandPairs * T) bail = true;
+        if (mr > L.rcap || mc > L.ccap) bail = true;
+        if (!ids && (long long)mr * tc > s.cand_pairs) bail = true;
         __syncthreads();
       };
       auto col_rank = [&](int32_t e) {  // CTA whose list holds candidate column e

@@ -6,16 +6,23 @@ namespace tsb {
 
 constexpr int kCandSlice = 4096;             // vertices per CTA the cluster size aims at
 constexpr size_t kCandSmem = 220 * 1024;     // dynamic shared memory a CTA may ask for
+constexpr size_t kCandPersistSmem = 200 * 1024;  // the same beside the persistent kernels' static part
 
 struct CandPlan {
   int cs = 0;               // CTAs of the cluster; 0: the state does not fit
   int32_t rpc = 0, cpc = 0; // rows and columns per CTA (multiples of 4)
   int32_t fav = 0;          // every c*w >= 0
   int64_t plus = 0;         // upper bound of c*w
+  int64_t pairs = 0;        // candidate pairs per CTA before a sweep is cheaper
   size_t smem = 0;
 };
 // Slices for a given cluster size within `limit` bytes of shared memory.
 CandPlan cand_slices(const ts_graph* g, int32_t problem, int32_t m, bool wide, int cs, size_t limit);
+// The same for a persistent (batched, served) solve; cs 0 when the pass does
+// not apply: a pinned sweep, or a state too large for the cluster.
+CandPlan cand_persist(const ts_graph* g, int32_t problem, int32_t m, bool wide, int32_t pass, int cs);
+// Cluster size of a persistent solve whose caller leaves it open.
+int cand_cluster(int32_t n);
 // The plain form's choice of cluster size.
 CandPlan cand_plan(const ts_graph* g, int32_t problem, int32_t m, bool wide);
 // `solver` points to a DevSolver<KeyT> (KeyT by `wide`).

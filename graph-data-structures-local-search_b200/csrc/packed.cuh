@@ -4,6 +4,7 @@
 #pragma once
 #include <cooperative_groups.h>
 
+#include "cand.cuh"
 #include "sweep.cuh"
 
 namespace tsb {
@@ -176,16 +177,21 @@ __device__ void slot_finish(const DevGraph& g, const DevSolver<KeyT>& s, BatchRe
 
 
 // Runs a solve's iterations up to `stop_at` with the CTAs of the calling
-// cluster: round-robin tiles, the leader merges the records over distributed
-// shared memory and applies the move.  Every CTA of the cluster calls it.
+// cluster: the candidate pass where the solve has it, else (and for the
+// iterations it leaves) round-robin tiles, the leader merging the records over
+// distributed shared memory and applying the move.  Every CTA of the cluster
+// calls it.
 template <int PROB, int ST, class KeyT>
 __device__ void cluster_iterate(const DevGraph& g, const DevSolver<KeyT>& s, long long stop_at,
-                                cooperative_groups::cluster_group& cl, TailShared& sh, CtaRec& s_rec) {
+                                cooperative_groups::cluster_group& cl, TailShared& sh, CtaRec& s_rec,
+                                CandShared<KeyT>& s_cand) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const unsigned rank = cl.block_rank(), cs = cl.num_blocks();
   const int tid = threadIdx.x;
   const int ntiles = s.n_row_blocks * s.n_chunks;
   const DevState* st = s.st;
   for (;;) {
+    if (s.cand_rpc > 0 && cand_run<PROB, ST, KeyT>(g, s, stop_at, LLONG_MAX, cl, s_cand, smem_raw) == kCandEnd) break;
     // every CTA reads the same state: the leader wrote it before the last barrier
     const long long it = __ldcg(&st->iter);
     if (__ldcg(&st->done) || it >= stop_at) break;

@@ -30,6 +30,7 @@
 #include <tuple>
 #include <vector>
 
+#include "cand.h"
 #include "packed.cuh"
 #include "ts_host.h"
 
@@ -59,6 +60,7 @@ serve_kernel(const ServeJobDev<KeyT>* __restrict__ jobs) {
   const unsigned rank = cl.block_rank(), cs = cl.num_blocks();
   __shared__ TailShared sh;
   __shared__ CtaRec s_rec;
+  __shared__ CandShared<KeyT> s_cand;
   __shared__ long long sc[kMaxTPB / 32];
   __shared__ int32_t s_cnt[kMaxTPB];
   const ServeJobDev<KeyT> J = jobs[blockIdx.x / cs];
@@ -67,7 +69,7 @@ serve_kernel(const ServeJobDev<KeyT>* __restrict__ jobs) {
     __threadfence();
   }
   cl.sync();
-  cluster_iterate<PROB, ST, KeyT>(J.g, J.s, J.stop_at < J.max_iter ? J.stop_at : J.max_iter, cl, sh, s_rec);
+  cluster_iterate<PROB, ST, KeyT>(J.g, J.s, J.stop_at < J.max_iter ? J.stop_at : J.max_iter, cl, sh, s_rec, s_cand);
   if (rank == 0) {
     const DevState* st = J.s.st;
     if (__ldcg(&st->done) || __ldcg(&st->iter) >= J.max_iter)
@@ -236,7 +238,13 @@ ts_status build_packed(Req& r, int32_t kind) {
   s.chunk_cols = tg.chunk_cols;
   s.n_chunks = tg.n_chunks;
   s.stage_bytes = tg.stage_bytes;
-  r.smem = tg.smem;
+  const CandPlan cp = cand_persist(r.g, r.p.problem, m, sizeof(KeyT) == 8, r.p.pass, r.cs);
+  s.cand_rpc = cp.cs ? cp.rpc : 0;
+  s.cand_cpc = cp.cpc;
+  s.cand_fav = cp.fav;
+  s.cand_plus = cp.plus;
+  s.cand_pairs = cp.pairs;
+  r.smem = std::max(tg.smem, cp.cs ? cp.smem : (size_t)0);
   s.P = (int64_t)m * delta;
   const int64_t entries = r.g->entries;
   const int64_t events = r.p.problem == P_MAXBS ? r.p.max_iter / r.p.piter + 1 : 0;
@@ -506,8 +514,9 @@ void ts_server::round() {
     size_t smem = 16;
     for (size_t q = 0; q < js.size(); q++) {
       Req& r = *js[q];
+      // seconds per iteration: the candidate pass, or the cluster's sweep
       const double per_cta = 5e9;
-      const double est = 6e-6 + (double)r.P / (per_cta * r.cs);
+      const double est = r.p.pass == TS_PASS_AUTO ? 6e-6 : 6e-6 + (double)r.P / (per_cta * r.cs);
       const int64_t k = std::max<int64_t>(4, std::min<int64_t>(1 << 16, (int64_t)(round_s / est)));
       r.granted += k;
       unsigned char* dst = static_cast<unsigned char*>(G.host) + rec * q;

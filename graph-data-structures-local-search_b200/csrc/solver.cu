@@ -437,7 +437,7 @@ struct ts_solver {
     s.fast_ecap = fast_ecap;
     s.n_slices = n_slices;
     s.w16 = w16;
-    s.cand_rpc = cand.rpc; s.cand_cpc = cand.cpc; s.cand_fav = cand.fav; s.cand_plus = cand.plus;
+    s.cand_rpc = cand.rpc; s.cand_cpc = cand.cpc; s.cand_fav = cand.fav; s.cand_plus = cand.plus; s.cand_pairs = cand.pairs;
     s.P = P;
     s.sol_in = sol_in.as<int32_t>(); s.sol_out = sol_out.as<int32_t>();
     s.vg_in = vg_in.as<KeyT>(); s.vg_out = vg_out.as<KeyT>();

@@ -113,6 +113,7 @@ struct DevSolver {
   int32_t cand_rpc, cand_cpc, cand_fav;
   int32_t guard;          // this launch runs only while DevState::owed > 0
   int64_t cand_plus;
+  int64_t cand_pairs;     // candidate pairs one CTA looks up before a sweep is cheaper
   int64_t P;
   int32_t* sol_in;
   int32_t* sol_out;

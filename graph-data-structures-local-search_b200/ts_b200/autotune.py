@@ -89,7 +89,7 @@ def _trial(problem: int, n: int, kind: str, cluster: int, jobs: int, iters: int,
 
 
 def autotune(buckets=DEFAULT_BUCKETS, kinds=("csr", "wswap", "csr-bb", "hash"), clusters=(1, 2, 4),
-             sweeps=(C.PASS_TILE, C.PASS_ROWS), jobs: int = 296, iters: int = 60, seed: int = 123,
+             sweeps=(C.PASS_TILE, C.PASS_ROWS, C.PASS_AUTO), jobs: int = 296, iters: int = 60, seed: int = 123,
              budget_s: float = 60.0) -> Table:
     """Times every candidate on the geometric middle of each bucket; each
     (problem, bucket) gets an equal share of `budget_s`, after which it keeps
