@@ -27,21 +27,21 @@ cand_kernel(const DevGraph g, const DevSolver<KeyT> s, long long budget) {
 }
 
 template <int PROB, int ST, class KeyT>
-cudaError_t configure(int cs, size_t smem, cudaStream_t st, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr) {
+cudaError_t configure(const CandPlan& p, cudaStream_t st, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr) {
   const void* fn = reinterpret_cast<const void*>(cand_kernel<PROB, ST, KeyT>);
-  cudaError_t e = allow_dyn_smem(fn, smem);
+  cudaError_t e = allow_dyn_smem(fn, p.smem);
   if (e != cudaSuccess) return e;
-  if (cs > 8) {
+  if (p.cs > 8) {
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
   }
   cfg = {};
-  cfg.gridDim = dim3((unsigned)cs);
-  cfg.blockDim = dim3(kCandTPB);
-  cfg.dynamicSmemBytes = smem;
+  cfg.gridDim = dim3((unsigned)p.cs);
+  cfg.blockDim = dim3((unsigned)p.threads);
+  cfg.dynamicSmemBytes = p.smem;
   cfg.stream = st;
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)cs;
+  attr[0].val.clusterDim.x = (unsigned)p.cs;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
@@ -51,19 +51,19 @@ cudaError_t configure(int cs, size_t smem, cudaStream_t st, cudaLaunchConfig_t& 
 
 template <int PROB, int ST, class KeyT>
 struct Launch {
-  static cudaError_t run(const DevGraph& g, const void* s, int cs, size_t smem, cudaStream_t st, long long budget) {
+  static cudaError_t run(const DevGraph& g, const void* s, const CandPlan& p, cudaStream_t st, long long budget) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
-    const cudaError_t e = configure<PROB, ST, KeyT>(cs, smem, st, cfg, attr);
+    const cudaError_t e = configure<PROB, ST, KeyT>(p, st, cfg, attr);
     if (e != cudaSuccess) return e;
     return cudaLaunchKernelEx(&cfg, cand_kernel<PROB, ST, KeyT>, g, *static_cast<const DevSolver<KeyT>*>(s), budget);
   }
-  // Clusters of cs CTAs the device can hold (0: none).
-  static int resident(int cs, size_t smem) {
+  // Clusters of the plan's size the device can hold (0: none).
+  static int resident(const CandPlan& p) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
     int n = 0;
-    if (configure<PROB, ST, KeyT>(cs, smem, nullptr, cfg, attr) != cudaSuccess ||
+    if (configure<PROB, ST, KeyT>(p, nullptr, cfg, attr) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, cand_kernel<PROB, ST, KeyT>, &cfg) != cudaSuccess) {
       cudaGetLastError();
       return 0;
@@ -100,8 +100,23 @@ CandPlan cand_slices(const ts_graph* g, int32_t problem, int32_t m, bool wide, i
   const int32_t delta = g->n - m;
   p.rpc = ((m + cs - 1) / cs + 3) & ~3;
   p.cpc = ((delta + cs - 1) / cs + 3) & ~3;
-  p.smem = cand_layout(g->n, p.rpc, p.cpc, wide ? 8 : 4, p.plus > 0).total;
-  if (p.smem <= limit) p.cs = cs;
+  const int kb = wide ? 8 : 4;
+  // Positions by vertex go to shared memory where they fit.
+  const int32_t vpc = ((g->n + cs - 1) / cs + 3) & ~3;
+  const bool map = p.plus > 0;
+  p.vpc = cand_layout(g->n, p.rpc, p.cpc, kb, vpc, map).total <= limit ? vpc : 0;
+  p.smem = cand_layout(g->n, p.rpc, p.cpc, kb, p.vpc, map).total;
+  p.threads = kCandTPB;
+  // Divisions by a slice are a multiplication by ceil(2^32 / slice), exact
+  // for up to 16 slices of fewer than 2^14.
+  const int32_t per[3] = {p.rpc, p.cpc, p.vpc};
+  bool exact = true;
+  for (int k = 0; k < 3; k++) {
+    if (!per[k]) continue;
+    p.inv[k] = (uint32_t)(((1ULL << 32) + per[k] - 1) / per[k]);
+    exact = exact && (uint64_t)cs * per[k] * per[k] < (1ULL << 32);
+  }
+  if (p.smem <= limit && exact) p.cs = cs;
   // Looking up 64 pairs a thread takes about as long as a small sweep launch.
   p.pairs = 64 * kCandTPB;
   return p;
@@ -117,27 +132,34 @@ CandPlan cand_persist(const ts_graph* g, int32_t problem, int32_t m, bool wide, 
   return p;
 }
 
-// One CTA while the batch has solves for every SM: per iteration one 256-thread
-// CTA against two took 4.5 against 4.2 us (MDP, n = 5,000) and 33 against 21 us
-// (Max Bisection, n = 3,000) -- less than twice as fast on twice the SMs.
-// Larger solves need the second CTA's shared memory.
+// One 256-thread CTA while the batch has solves for every SM: per iteration one
+// CTA against four took 2.7 against 3.4 us (MDP, n = 5,000), 12.9 against 10.0
+// us (Max Bisection, n = 5,000) and 22 against 11.7 us (n = 12,000) -- less
+// than twice as fast on four times the SMs.  Larger solves need the other
+// CTAs' shared memory.
 int cand_cluster(int32_t n) { return n <= 6144 ? 1 : (n <= 16384 ? 2 : 4); }
 
 CandPlan cand_plan(const ts_graph* g, int32_t problem, int32_t m, bool wide) {
-  // A CTA scans about 4,000 positions in the time of one cluster barrier;
-  // more CTAs also share the candidates' rows.
-  int cs = 1;
-  while (cs < kCandMaxCluster && (int64_t)cs * kCandSlice < g->n) cs *= 2;
+  // Max Bisection spends most of an iteration on candidate rows, which more
+  // CTAs share; an MDP iteration mostly scans and applies, and one CTA needs
+  // no cluster barriers.  1 / 8 / 16 CTAs, us per iteration: MDP ER n = 2,000
+  // 2.5 / 3.5 / 3.7; dense n = 2,000 7.8 / 8.6 / 10.4; bisection n = 5,000
+  // 14.5 / 10.1 / 10.4, n = 30,011 16.8 / 10.6 / 10.3, n = 100,000 - / 16.5 /
+  // 13.9.
+  const int n = g->n;
+  const bool edges = problem == P_MAXBS || g->neg_w;
+  int cs = edges ? (n <= 4096 ? 1 : (n <= 32768 ? 8 : 16)) : (n <= 8192 ? 1 : (n <= 32768 ? 4 : 16));
   for (; cs <= kCandMaxCluster; cs *= 2) {
     CandPlan p = cand_slices(g, problem, m, wide, cs, kCandSmem);
-    if (p.cs && by_kind(problem, g->kind, wide, [&](auto l) { return decltype(l)::resident(cs, p.smem); }) > 0) return p;
+    p.threads = n <= 1024 ? 256 : kCandTPB;
+    if (p.cs && by_kind(problem, g->kind, wide, [&](auto l) { return decltype(l)::resident(p); }) > 0) return p;
   }
   return CandPlan{};
 }
 
-cudaError_t launch_cand(int32_t problem, int kind, bool wide, const DevGraph& g, const void* solver, int cs, size_t smem,
+cudaError_t launch_cand(int32_t problem, int kind, bool wide, const DevGraph& g, const void* solver, const CandPlan& plan,
                         cudaStream_t st, long long budget) {
-  return by_kind(problem, kind, wide, [&](auto l) { return decltype(l)::run(g, solver, cs, smem, st, budget); });
+  return by_kind(problem, kind, wide, [&](auto l) { return decltype(l)::run(g, solver, plan, st, budget); });
 }
 
 }  // namespace tsb

@@ -4,13 +4,15 @@
 
 namespace tsb {
 
-constexpr int kCandSlice = 4096;             // vertices per CTA the cluster size aims at
 constexpr size_t kCandSmem = 220 * 1024;     // dynamic shared memory a CTA may ask for
 constexpr size_t kCandPersistSmem = 200 * 1024;  // the same beside the persistent kernels' static part
 
 struct CandPlan {
   int cs = 0;               // CTAs of the cluster; 0: the state does not fit
+  int threads = 0;          // per CTA
   int32_t rpc = 0, cpc = 0; // rows and columns per CTA (multiples of 4)
+  int32_t vpc = 0;          // vertices per CTA of the position slice; 0: positions stay in HBM
+  uint32_t inv[3] = {0, 0, 0};  // ceil(2^32 / slice): rows, columns, vertices
   int32_t fav = 0;          // every c*w >= 0
   int64_t plus = 0;         // upper bound of c*w
   int64_t pairs = 0;        // candidate pairs per CTA before a sweep is cheaper
@@ -26,7 +28,7 @@ int cand_cluster(int32_t n);
 // The plain form's choice of cluster size.
 CandPlan cand_plan(const ts_graph* g, int32_t problem, int32_t m, bool wide);
 // `solver` points to a DevSolver<KeyT> (KeyT by `wide`).
-cudaError_t launch_cand(int32_t problem, int kind, bool wide, const DevGraph& g, const void* solver, int cs, size_t smem,
+cudaError_t launch_cand(int32_t problem, int kind, bool wide, const DevGraph& g, const void* solver, const CandPlan& plan,
                         cudaStream_t st, long long budget);
 
 }  // namespace tsb

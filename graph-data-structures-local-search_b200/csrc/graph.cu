@@ -103,17 +103,22 @@ __global__ void k_pack_adj(int64_t N, const unsigned long long* __restrict__ key
 // (out[0]); out[1] != 0 when some weight is negative; out[2] = max |w| (the
 // WSwap matrix holds 16-bit weights when it fits).
 __global__ void k_max_wdeg(int32_t n, const int64_t* __restrict__ rowptr,
-                           const int2* __restrict__ adj, unsigned long long* __restrict__ out) {
+                           const int2* __restrict__ adj, unsigned long long* __restrict__ out,
+                           int2* __restrict__ wrange) {
   for (int32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
     unsigned long long s = 0, mx = 0;
     bool neg = false;
+    int2 wr = make_int2(0, 0);  // of the row's weights and 0
     for (int64_t k = rowptr[r]; k < rowptr[r + 1]; k++) {
       int32_t x = adj[k].y;
       const unsigned long long a = (unsigned long long)(x < 0 ? -(long long)x : (long long)x);
       s += a;
       mx = a > mx ? a : mx;
       neg |= x < 0;
+      wr.x = x < wr.x ? x : wr.x;
+      wr.y = x > wr.y ? x : wr.y;
     }
+    wrange[r] = wr;
     atomicMax(out, s);
     if (neg) atomicMax(out + 1, 1ull);
     if (mx) atomicMax(out + 2, mx);
@@ -334,9 +339,10 @@ static ts_status build_graph(ts_graph* G, int64_t E, const int32_t* d_u, const i
   vals_alt.release();
   tmp.release();
   TS_CUDA(cudaMemsetAsync(cnt.p, 0, 3 * sizeof(unsigned long long), st));
+  if ((s = G->wrange.alloc(sizeof(int2) * (size_t)(n > 0 ? n : 1), "alloc row weight ranges")) != TS_OK) return s;
   if (n > 0) {
     k_max_wdeg<<<blocks_for(n), kTPB, 0, st>>>(n, G->rowptr.as<int64_t>(), G->adj.as<int2>(),
-                                               cnt.as<unsigned long long>());
+                                               cnt.as<unsigned long long>(), G->wrange.as<int2>());
     TS_CUDA(cudaGetLastError());
   }
   unsigned long long mw[3] = {0, 0, 0};

@@ -241,6 +241,8 @@ ts_status build_packed(Req& r, int32_t kind) {
   const CandPlan cp = cand_persist(r.g, r.p.problem, m, sizeof(KeyT) == 8, r.p.pass, r.cs);
   s.cand_rpc = cp.cs ? cp.rpc : 0;
   s.cand_cpc = cp.cpc;
+  s.cand_vpc = cp.vpc;
+  for (int k = 0; k < 3; k++) s.cand_inv[k] = cp.inv[k];
   s.cand_fav = cp.fav;
   s.cand_plus = cp.plus;
   s.cand_pairs = cp.pairs;

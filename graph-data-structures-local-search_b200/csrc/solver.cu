@@ -437,7 +437,9 @@ struct ts_solver {
     s.fast_ecap = fast_ecap;
     s.n_slices = n_slices;
     s.w16 = w16;
-    s.cand_rpc = cand.rpc; s.cand_cpc = cand.cpc; s.cand_fav = cand.fav; s.cand_plus = cand.plus; s.cand_pairs = cand.pairs;
+    s.cand_rpc = cand.rpc; s.cand_cpc = cand.cpc; s.cand_vpc = cand.vpc;
+    for (int k = 0; k < 3; k++) s.cand_inv[k] = cand.inv[k];
+    s.cand_fav = cand.fav; s.cand_plus = cand.plus; s.cand_pairs = cand.pairs;
     s.P = P;
     s.sol_in = sol_in.as<int32_t>(); s.sol_out = sol_out.as<int32_t>();
     s.vg_in = vg_in.as<KeyT>(); s.vg_out = vg_out.as<KeyT>();
@@ -822,7 +824,7 @@ ts_status enqueue_launches(ts_solver* s, int64_t iters) {
   const DevSolver<int32_t> d4 = s->dev<int32_t>();
   const void* d = s->wide ? static_cast<const void*>(&d8) : &d4;
   for (; iters > 0; iters -= kCandLaunchIters) {
-    const cudaError_t e = launch_cand(s->p.problem, s->g->kind, s->wide, g, d, s->cand.cs, s->cand.smem, s->g->stream,
+    const cudaError_t e = launch_cand(s->p.problem, s->g->kind, s->wide, g, d, s->cand, s->g->stream,
                                       std::min<int64_t>(iters, kCandLaunchIters));
     if (e != cudaSuccess) return cuda_fail(e, "candidate kernel launch");
   }

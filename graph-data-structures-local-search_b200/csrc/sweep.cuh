@@ -79,12 +79,14 @@ __host__ __device__ inline int rows_of(int st) {
 template <class KeyT> struct KeyLim;
 template <> struct KeyLim<int32_t> {
   static constexpr int32_t none = INT32_MIN;
+  static constexpr int32_t high = INT32_MAX;
   __device__ static int32_t clampD(long long d) {
     return d > INT32_MAX ? INT32_MAX : (d < INT32_MIN + 1 ? INT32_MIN + 1 : (int32_t)d);
   }
 };
 template <> struct KeyLim<long long> {
   static constexpr long long none = LLONG_MIN;
+  static constexpr long long high = LLONG_MAX;
   __device__ static long long clampD(long long d) { return d; }
 };
 

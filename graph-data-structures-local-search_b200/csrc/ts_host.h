@@ -79,7 +79,7 @@ struct ts_graph {
   int64_t max_abs_w = 0;  // largest |w| of an entry
   int64_t wpr = 0;
   int64_t hash_slots = 0;
-  tsb::DevBuf rowptr, adj, bits, hoff, hkey, hval, rev;
+  tsb::DevBuf rowptr, adj, bits, hoff, hkey, hval, rev, wrange;
   // Host copy of the CSR row pointers/degrees (for footprint planning and the
   // solver's staging budgets); small: n+1 int64.
   std::vector<int64_t> h_rowptr;
@@ -96,10 +96,11 @@ struct ts_graph {
     g.hkey = hkey.as<int32_t>();
     g.hval = hval.as<int32_t>();
     g.rev = rev.as<int64_t>();
+    g.wrange = wrange.as<int2>();
     return g;
   }
   int64_t device_bytes() const {
-    return (int64_t)(rowptr.bytes + adj.bytes + bits.bytes + hoff.bytes + hkey.bytes + hval.bytes + rev.bytes);
+    return (int64_t)(rowptr.bytes + adj.bytes + bits.bytes + hoff.bytes + hkey.bytes + hval.bytes + rev.bytes + wrange.bytes);
   }
   mutable int64_t deg90 = -1;  // 90th-percentile degree, computed on first use
 };

@@ -46,6 +46,7 @@ struct DevGraph {
   const int64_t* hoff;
   const int32_t* hkey;  // Hash: per-vertex tables, keys (neighbour id, -1 empty) ...
   const int32_t* hval;  // ... and weights, same slots
+  const int2* wrange;   // smallest and largest weight of every row (0 included)
   const int64_t* rev;   // CSR only: index of the mirrored entry (z->y) of every entry (y->z)
 };
 
@@ -107,10 +108,11 @@ struct DevSolver {
   // WSwap: 1 when the matrix holds 16-bit weights (every |w| <= 32767), read
   // through W as int16_t; 0: 32-bit.
   int32_t w16;
-  // Candidate pass (cand.cuh): CTAs' slices of rows and columns (0: off),
-  // whether every c*w >= 0 (Max Bisection without negative weights) and the
+  // Candidate pass (cand.cuh): CTAs' slices of rows and columns (0: off) and
+  // of the positions by vertex (0: read from HBM), whether every c*w >= 0 (Max Bisection without negative weights) and the
   // upper bound of c*w over the graph's edges.
-  int32_t cand_rpc, cand_cpc, cand_fav;
+  int32_t cand_rpc, cand_cpc, cand_vpc, cand_fav;
+  uint32_t cand_inv[3];   // ceil(2^32 / slice): rows, columns, vertices
   int32_t guard;          // this launch runs only while DevState::owed > 0
   int64_t cand_plus;
   int64_t cand_pairs;     // candidate pairs one CTA looks up before a sweep is cheaper
