@@ -201,42 +201,101 @@ inline int grid_for(int64_t n, int tpb = kInitTPB) {
   return (int)b;
 }
 
+// Start positions: ascending ids per side (initialSolution,
+// GPU-MDP-CSR.cu:479-500), from a flag per vertex.  A block places kPlace
+// vertices; the inside ones before them come from the blocks' counts.
+constexpr int kPlace = 1024;
+__global__ void __launch_bounds__(kPlace) k_count_inside(int32_t n, const uint8_t* __restrict__ inside, int32_t* __restrict__ count) {
+  const int32_t v = blockIdx.x * kPlace + threadIdx.x;
+  const int c = __syncthreads_count(v < n && inside[v]);
+  if (threadIdx.x == 0) count[blockIdx.x] = c;
+}
 template <class KeyT>
-__global__ void k_init_mdp(const DevGraph g, const DevSolver<KeyT> s, unsigned long long* obj2) {
-  // calculateVertexGain (GPU-MDP-CSR.cu:502-519): vg[z] += w for z in N(S).
-  for (int32_t i = blockIdx.x; i < s.m; i += gridDim.x) {
-    const int32_t u = s.sol_in[i];
-    unsigned long long acc = 0;
-    for (long long k = g.rowptr[u] + threadIdx.x; k < g.rowptr[u + 1]; k += blockDim.x) {
-      const int2 e = g.adj[k];
-      const int32_t p = s.pos[e.x];
-      atomic_add_key(vg_at(s, p), (KeyT)e.y);
-      if (p < s.m) acc += (unsigned long long)(long long)e.y;
-    }
-    if (acc) atomicAdd(obj2, acc);
+__global__ void __launch_bounds__(kPlace)
+k_place(const DevSolver<KeyT> s, const uint8_t* __restrict__ inside, const int32_t* __restrict__ count) {
+  __shared__ int32_t part[kPlace / 32], before_me;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int32_t v = blockIdx.x * kPlace + tid;
+  const bool in = v < s.n && inside[v];
+  const unsigned b = __ballot_sync(0xffffffffu, in);
+  int32_t sum = 0;  // inside vertices of the earlier blocks
+  for (int k = tid; k < (int)blockIdx.x; k += kPlace) sum += count[k];
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if (tid == 0) before_me = 0;
+  __syncthreads();
+  if (lane == 0) {
+    part[warp] = __popc(b);
+    if (sum) atomicAdd(&before_me, sum);
+  }
+  __syncthreads();
+  int32_t x = before_me + __popc(b & ((1u << lane) - 1u));
+  for (int w = 0; w < warp; w++) x += part[w];
+  if (v < s.n) {
+    const int32_t y = v - x;
+    s.pos[v] = in ? x : s.m + y;
+    if (in) { s.sol_in[x] = v; s.vg_in[x] = 0; s.tab_in[x] = 0; }
+    else { s.sol_out[y] = v; s.vg_out[y] = 0; s.tab_out[y] = 0; }
+  }
+  if (blockIdx.x == 0 && tid < s.ldc - s.delta) {  // padding columns
+    const int32_t y = s.delta + tid;
+    s.sol_out[y] = 0; s.vg_out[y] = 0; s.tab_out[y] = 0;
+  }
+}
+
+// Sum of a block's values into *out: one atomic per block.
+__device__ __forceinline__ void add_block(long long v, unsigned long long* out) {
+  __shared__ long long part[kInitTPB / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kInitTPB / 32; w++) v += part[w];
+    if (v) atomicAdd(out, (unsigned long long)v);
   }
 }
 
 template <class KeyT>
+__global__ void k_init_mdp(const DevGraph g, const DevSolver<KeyT> s, unsigned long long* obj2) {
+  // calculateVertexGain (GPU-MDP-CSR.cu:502-519): vg[z] += w for z in N(S).
+  long long acc = 0;
+  for (int32_t i = blockIdx.x; i < s.m; i += gridDim.x) {
+    const int32_t u = s.sol_in[i];
+    for (long long k = g.rowptr[u] + threadIdx.x; k < g.rowptr[u + 1]; k += blockDim.x) {
+      const int2 e = g.adj[k];
+      const int32_t p = s.pos[e.x];
+      atomic_add_key(vg_at(s, p), (KeyT)e.y);
+      if (p < s.m) acc += e.y;
+    }
+  }
+  add_block(acc, obj2);
+}
+
+// The kernels below take a warp per row: a thread per row walked the rows of
+// hubs (5,000 entries) and of dense graphs one load after another.  Measured
+// with the host work that the device now does (positions, state by vertex):
+// Chung-Lu n = 200,000 init 360 -> 110 us, result 1,200 -> 300, state 2,800 ->
+// 1,150 (4 MB of copies); dense n = 2,000 result 545 -> 110.
+template <class KeyT>
 __global__ void k_init_maxbs(const DevGraph g, const DevSolver<KeyT> s, unsigned long long* cut) {
   // computeGainsFromScratch / computeFitnessFromScratch (GPU-MAXBS-CSR.cu:197-219).
-  for (int32_t z = blockIdx.x * blockDim.x + threadIdx.x; z < s.n; z += gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  long long c = 0;
+  for (int32_t z = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; z < s.n; z += (gridDim.x * blockDim.x) >> 5) {
     const int32_t pz = s.pos[z];
     const bool side = pz < s.m;
-    long long same = 0, opp = 0;
-    unsigned long long c = 0;
-    for (long long k = g.rowptr[z]; k < g.rowptr[z + 1]; k++) {
+    long long gain = 0;  // same side minus opposite
+    for (long long k = g.rowptr[z] + lane; k < g.rowptr[z + 1]; k += 32) {
       const int2 e = g.adj[k];
       const bool sy = s.pos[e.x] < s.m;
-      if (sy == side) same += e.y;
-      else {
-        opp += e.y;
-        if (e.x > z) c += (unsigned long long)(long long)e.y;
-      }
+      gain += sy == side ? e.y : -e.y;
+      if (sy != side && e.x > z) c += e.y;
     }
-    *vg_at(s, pz) = (KeyT)(same - opp);
-    if (c) atomicAdd(cut, c);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) gain += __shfl_xor_sync(0xffffffffu, gain, o);
+    if (lane == 0) *vg_at(s, pz) = (KeyT)gain;
   }
+  add_block(c, cut);
 }
 
 // W[i][j] = w(sol_in[i], sol_out[j]) (calculateEdgeGain, GPU-MDP-WSwap.cu:607-626),
@@ -263,20 +322,38 @@ __global__ void k_init_cpos(const DevGraph g, const DevSolver<KeyT> s) {
     s.cpos[k] = s.pos[g.adj[k].x];
 }
 
-// Objective of a set / bisection given per-vertex flags (1 = inside / side 0).
+// Objective of a set / bisection given per-vertex flags (1 = inside / side 0):
+// MDP twice the weight inside (rows of inside vertices only), else the cut.
 __global__ void k_objective(const DevGraph g, int32_t problem, const uint8_t* in,
                             unsigned long long* out) {
-  for (int32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < g.n; a += gridDim.x * blockDim.x) {
-    unsigned long long acc = 0;
-    for (long long k = g.rowptr[a]; k < g.rowptr[a + 1]; k++) {
+  const int lane = threadIdx.x & 31;
+  long long acc = 0;
+  for (int32_t a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; a < g.n; a += (gridDim.x * blockDim.x) >> 5) {
+    const uint8_t side = in[a];
+    if (problem == P_MDP && !side) continue;
+    for (long long k = g.rowptr[a] + lane; k < g.rowptr[a + 1]; k += 32) {
       const int2 e = g.adj[k];
       if (problem == P_MDP) {
-        if (in[a] && in[e.x]) acc += (unsigned long long)(long long)e.y;
-      } else if (e.x > a && in[a] != in[e.x]) {
-        acc += (unsigned long long)(long long)e.y;
+        if (in[e.x]) acc += e.y;
+      } else if (e.x > a && side != in[e.x]) {
+        acc += e.y;
       }
     }
-    if (acc) atomicAdd(out, acc);
+  }
+  add_block(acc, out);
+}
+
+// State by vertex for the caller: ids in position order, stamps and
+// contributions by vertex id.
+template <class KeyT>
+__global__ void k_state(const DevSolver<KeyT> s, int32_t* __restrict__ sol, int32_t* __restrict__ tab,
+                        long long* __restrict__ vg) {
+  for (int32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < s.n; p += gridDim.x * blockDim.x) {
+    const bool in = p < s.m;
+    const int32_t q = in ? p : p - s.m, v = (in ? s.sol_in : s.sol_out)[q];
+    sol[p] = v;
+    tab[v] = (in ? s.tab_in : s.tab_out)[q];
+    vg[v] = (long long)(in ? s.vg_in : s.vg_out)[q];
   }
 }
 
@@ -404,7 +481,7 @@ struct ts_solver {
   int32_t num_pert = 1;
   int64_t log_cap = 0, trace_cap = 0;
   int64_t window_events = 0;
-  DevBuf sol_in, sol_out, vg_in, vg_out, tab_in, tab_out, pos, W, cpos, st, recs, movelog, trace, draws;
+  DevBuf sol_in, sol_out, vg_in, vg_out, tab_in, tab_out, pos, W, cpos, st, recs, movelog, trace, draws, work;
   std::mt19937 rng;
   std::vector<long long> host_draws;  // every perturbation event drawn so far, k draws each
   int64_t events_drawn = 0;
@@ -510,31 +587,38 @@ ts_status prepare_draws(ts_solver* s, int64_t iters_ahead) {
   return TS_OK;
 }
 
+// Device scratch of the calls outside the iterations, kept with the solver: a
+// sum, the blocks' counts and a flag per vertex (init, result), or ids, stamps
+// and contributions (state, the largest).
+ts_status scratch(ts_solver* s, unsigned char** p) {
+  if (!s->work.p) {
+    const ts_status rc = s->work.alloc(16 * (size_t)s->n + 512, "alloc solver scratch");
+    if (rc != TS_OK) return rc;
+  }
+  *p = s->work.as<unsigned char>();
+  return TS_OK;
+}
+
 template <class KeyT>
 ts_status init_device(ts_solver* s, const std::vector<uint8_t>& inside) {
   const int32_t n = s->n, m = s->m;
   cudaStream_t st = s->g->stream;
-  std::vector<int32_t> sin(m), sout(s->ldc, 0), pos(n);
-  int32_t x = 0, y = 0;
-  for (int32_t v = 0; v < n; v++) {  // initialSolution: ascending ids per side
-    if (inside[v]) { sin[x] = v; pos[v] = x; x++; }
-    else { sout[y] = v; pos[v] = m + y; y++; }
-  }
-  TS_CUDA(cudaMemcpyAsync(s->sol_in.p, sin.data(), sizeof(int32_t) * m, cudaMemcpyHostToDevice, st));
-  TS_CUDA(cudaMemcpyAsync(s->sol_out.p, sout.data(), sizeof(int32_t) * s->ldc, cudaMemcpyHostToDevice, st));
-  TS_CUDA(cudaMemcpyAsync(s->pos.p, pos.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, st));
-  TS_CUDA(cudaMemsetAsync(s->vg_in.p, 0, s->vg_in.bytes, st));
-  TS_CUDA(cudaMemsetAsync(s->vg_out.p, 0, s->vg_out.bytes, st));
-  TS_CUDA(cudaMemsetAsync(s->tab_in.p, 0, s->tab_in.bytes, st));
-  TS_CUDA(cudaMemsetAsync(s->tab_out.p, 0, s->tab_out.bytes, st));
-  DevBuf acc;
+  const int blocks = (n + kPlace - 1) / kPlace;
+  const size_t counts = 256, flags = counts + 4 * (size_t)blocks;
+  unsigned char* w = nullptr;
   ts_status rc;
-  if ((rc = acc.alloc(sizeof(unsigned long long), "alloc")) != TS_OK) return rc;
-  TS_CUDA(cudaMemsetAsync(acc.p, 0, sizeof(unsigned long long), st));
+  if ((rc = scratch(s, &w)) != TS_OK) return rc;
+  auto* acc = reinterpret_cast<unsigned long long*>(w);
+  auto* count = reinterpret_cast<int32_t*>(w + counts);
   DevSolver<KeyT> d = s->dev<KeyT>();
   DevGraph g = s->g->dev();
-  if (s->p.problem == P_MDP) k_init_mdp<KeyT><<<grid_for((int64_t)m * 32), kInitTPB, 0, st>>>(g, d, acc.as<unsigned long long>());
-  else k_init_maxbs<KeyT><<<grid_for(n), kInitTPB, 0, st>>>(g, d, acc.as<unsigned long long>());
+  TS_CUDA(cudaMemcpyAsync(w + flags, inside.data(), (size_t)n, cudaMemcpyHostToDevice, st));
+  TS_CUDA(cudaMemsetAsync(acc, 0, sizeof(unsigned long long), st));
+  k_count_inside<<<blocks, kPlace, 0, st>>>(n, w + flags, count);
+  k_place<KeyT><<<blocks, kPlace, 0, st>>>(d, w + flags, count);
+  TS_CUDA(cudaGetLastError());
+  if (s->p.problem == P_MDP) k_init_mdp<KeyT><<<grid_for((int64_t)m * 32), kInitTPB, 0, st>>>(g, d, acc);
+  else k_init_maxbs<KeyT><<<grid_for((int64_t)n * 32), kInitTPB, 0, st>>>(g, d, acc);
   TS_CUDA(cudaGetLastError());
   if (s->g->kind == S_WSWAP) {
     TS_CUDA(cudaMemsetAsync(s->W.p, 0, s->W.bytes, st));
@@ -546,7 +630,7 @@ ts_status init_device(ts_solver* s, const std::vector<uint8_t>& inside) {
     TS_CUDA(cudaGetLastError());
   }
   unsigned long long obj = 0;
-  TS_CUDA(cudaMemcpyAsync(&obj, acc.p, sizeof(obj), cudaMemcpyDeviceToHost, st));
+  TS_CUDA(cudaMemcpyAsync(&obj, acc, sizeof(obj), cudaMemcpyDeviceToHost, st));
   TS_CUDA(cudaStreamSynchronize(st));
   long long objective = (long long)obj;
   if (s->p.problem == P_MDP) objective /= 2;
@@ -558,17 +642,16 @@ ts_status init_device(ts_solver* s, const std::vector<uint8_t>& inside) {
 
 ts_status objective_of(ts_solver* s, const std::vector<uint8_t>& inside, long long* out) {
   cudaStream_t st = s->g->stream;
-  DevBuf flags, acc;
+  unsigned char* w = nullptr;
   ts_status rc;
-  if ((rc = flags.alloc(s->n, "alloc")) != TS_OK) return rc;
-  if ((rc = acc.alloc(sizeof(unsigned long long), "alloc")) != TS_OK) return rc;
-  TS_CUDA(cudaMemcpyAsync(flags.p, inside.data(), s->n, cudaMemcpyHostToDevice, st));
-  TS_CUDA(cudaMemsetAsync(acc.p, 0, sizeof(unsigned long long), st));
-  k_objective<<<grid_for(s->n), kInitTPB, 0, st>>>(s->g->dev(), s->p.problem, flags.as<uint8_t>(),
-                                                   acc.as<unsigned long long>());
+  if ((rc = scratch(s, &w)) != TS_OK) return rc;
+  auto* acc = reinterpret_cast<unsigned long long*>(w);
+  TS_CUDA(cudaMemcpyAsync(w + 256, inside.data(), s->n, cudaMemcpyHostToDevice, st));
+  TS_CUDA(cudaMemsetAsync(acc, 0, sizeof(unsigned long long), st));
+  k_objective<<<grid_for((int64_t)s->n * 32), kInitTPB, 0, st>>>(s->g->dev(), s->p.problem, w + 256, acc);
   TS_CUDA(cudaGetLastError());
   unsigned long long v = 0;
-  TS_CUDA(cudaMemcpyAsync(&v, acc.p, sizeof(v), cudaMemcpyDeviceToHost, st));
+  TS_CUDA(cudaMemcpyAsync(&v, acc, sizeof(v), cudaMemcpyDeviceToHost, st));
   TS_CUDA(cudaStreamSynchronize(st));
   long long r = (long long)v;
   if (s->p.problem == P_MDP) r /= 2;
@@ -992,37 +1075,22 @@ ts_status ts_solver_state(ts_solver* s, int32_t* sol, int32_t* pos, int32_t* tab
   if (!s->initialized) { set_error("ts_solver_state: call ts_solver_init first"); return TS_ERR_STATE; }
   TS_CUDA(cudaSetDevice(s->g->device));
   cudaStream_t st = s->g->stream;
-  const int32_t n = s->n, m = s->m, d = s->delta;
-  std::vector<int32_t> sin(m), sout(s->ldc), tin(m), tout(s->ldc), p(n);
-  std::vector<long long> vin(m), vout(s->ldc);
-  TS_CUDA(cudaMemcpyAsync(sin.data(), s->sol_in.p, 4 * (size_t)m, cudaMemcpyDeviceToHost, st));
-  TS_CUDA(cudaMemcpyAsync(sout.data(), s->sol_out.p, 4 * (size_t)s->ldc, cudaMemcpyDeviceToHost, st));
-  TS_CUDA(cudaMemcpyAsync(tin.data(), s->tab_in.p, 4 * (size_t)m, cudaMemcpyDeviceToHost, st));
-  TS_CUDA(cudaMemcpyAsync(tout.data(), s->tab_out.p, 4 * (size_t)s->ldc, cudaMemcpyDeviceToHost, st));
-  TS_CUDA(cudaMemcpyAsync(p.data(), s->pos.p, 4 * (size_t)n, cudaMemcpyDeviceToHost, st));
-  if (s->wide) {
-    TS_CUDA(cudaMemcpyAsync(vin.data(), s->vg_in.p, 8 * (size_t)m, cudaMemcpyDeviceToHost, st));
-    TS_CUDA(cudaMemcpyAsync(vout.data(), s->vg_out.p, 8 * (size_t)s->ldc, cudaMemcpyDeviceToHost, st));
-    TS_CUDA(cudaStreamSynchronize(st));
-  } else {
-    std::vector<int32_t> a(m), b(s->ldc);
-    TS_CUDA(cudaMemcpyAsync(a.data(), s->vg_in.p, 4 * (size_t)m, cudaMemcpyDeviceToHost, st));
-    TS_CUDA(cudaMemcpyAsync(b.data(), s->vg_out.p, 4 * (size_t)s->ldc, cudaMemcpyDeviceToHost, st));
-    TS_CUDA(cudaStreamSynchronize(st));
-    for (int32_t i = 0; i < m; i++) vin[i] = a[i];
-    for (int32_t j = 0; j < s->ldc; j++) vout[j] = b[j];
-  }
-  for (int32_t i = 0; i < m; i++) {
-    if (sol) sol[i] = sin[i];
-    if (tab) tab[sin[i]] = tin[i];
-    if (vg) vg[sin[i]] = vin[i];
-  }
-  for (int32_t j = 0; j < d; j++) {
-    if (sol) sol[m + j] = sout[j];
-    if (tab) tab[sout[j]] = tout[j];
-    if (vg) vg[sout[j]] = vout[j];
-  }
-  if (pos) std::memcpy(pos, p.data(), 4 * (size_t)n);
+  const size_t n = (size_t)s->n;
+  const size_t at_tab = 8 * n, at_sol = 12 * n;  // contributions first: 8-byte aligned
+  unsigned char* w = nullptr;
+  ts_status rc;
+  if ((rc = scratch(s, &w)) != TS_OK) return rc;
+  auto* d_vg = reinterpret_cast<long long*>(w);
+  auto* d_tab = reinterpret_cast<int32_t*>(w + at_tab);
+  auto* d_sol = reinterpret_cast<int32_t*>(w + at_sol);
+  if (s->wide) k_state<long long><<<grid_for(s->n), kInitTPB, 0, st>>>(s->dev<long long>(), d_sol, d_tab, d_vg);
+  else k_state<int32_t><<<grid_for(s->n), kInitTPB, 0, st>>>(s->dev<int32_t>(), d_sol, d_tab, d_vg);
+  TS_CUDA(cudaGetLastError());
+  if (sol) TS_CUDA(cudaMemcpyAsync(sol, d_sol, 4 * n, cudaMemcpyDeviceToHost, st));
+  if (pos) TS_CUDA(cudaMemcpyAsync(pos, s->pos.p, 4 * n, cudaMemcpyDeviceToHost, st));
+  if (tab) TS_CUDA(cudaMemcpyAsync(tab, d_tab, 4 * n, cudaMemcpyDeviceToHost, st));
+  if (vg) TS_CUDA(cudaMemcpyAsync(vg, d_vg, 8 * n, cudaMemcpyDeviceToHost, st));
+  TS_CUDA(cudaStreamSynchronize(st));
   return TS_OK;
 }
 
