@@ -35,6 +35,72 @@ ts_status cuda_fail(cudaError_t e, const char* what) {
   return e == cudaErrorMemoryAllocation ? TS_ERR_OUT_OF_MEMORY : TS_ERR_CUDA;
 }
 
+namespace {
+constexpr int kMaxDevices = 64;
+struct TempPool {
+  cudaMemPool_t pool = nullptr;
+  bool tried = false;
+  int users = 0;
+};
+std::mutex g_temp_mu;
+TempPool g_temp[kMaxDevices];
+
+// The current device's pool; nullptr where there is none (temporaries are then
+// ordinary stream-ordered allocations of the device's default pool).
+cudaMemPool_t temp_pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+  std::lock_guard<std::mutex> lock(g_temp_mu);
+  TempPool& t = g_temp[dev];
+  if (!t.tried) {
+    t.tried = true;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    uint64_t keep = kTempKeep;
+    if (cudaMemPoolCreate(&t.pool, &props) != cudaSuccess) {
+      t.pool = nullptr;
+      cudaGetLastError();
+    } else {
+      cudaMemPoolSetAttribute(t.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+  }
+  return t.pool;
+}
+}  // namespace
+
+cudaError_t temp_alloc(void** p, size_t bytes, cudaStream_t st) {
+  *p = nullptr;
+  const cudaMemPool_t pool = temp_pool();
+  for (int attempt = 0;; attempt++) {
+    const cudaError_t e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMallocAsync(p, bytes, st);
+    if (e != cudaErrorMemoryAllocation || attempt) return e;
+    cudaGetLastError();
+    temp_trim();
+  }
+}
+void temp_free(void* p, cudaStream_t st) {
+  if (p) cudaFreeAsync(p, st);
+}
+void temp_trim() {
+  const cudaMemPool_t pool = temp_pool();
+  if (!pool) return;
+  cudaDeviceSynchronize();  // frees still queued on a stream
+  cudaMemPoolTrimTo(pool, 0);
+}
+void temp_users(int device, int change) {
+  bool last = false;
+  if (device < 0 || device >= kMaxDevices) return;
+  {
+    std::lock_guard<std::mutex> lock(g_temp_mu);
+    g_temp[device].users += change;
+    last = change < 0 && g_temp[device].users == 0 && g_temp[device].pool;
+  }
+  if (last) cudaMemPoolTrimTo(g_temp[device].pool, kTempIdle);
+}
+
 cudaError_t allow_dyn_smem(const void* fn, size_t smem) {
   // The default limit is 48 KB minus the kernel's static shared memory, so
   // even a request below 48 KB may need the attribute raised.
@@ -58,9 +124,10 @@ inline int blocks_for(int64_t n, int tpb = kTPB) {
   return (int)b;
 }
 
-// Directed entries: 2 per edge ((u,v) at 2e, (v,u) at 2e+1), key = row<<32|col.
+// Directed entries: 2 per edge ((u,v) at 2e, (v,u) at 2e+1), key = row<<cb|col
+// with cb the bits of a column, so that the sort has no idle bits to pass over.
 // Dropped self-loops and out-of-range endpoints get row n (sorted past the end).
-__global__ void k_make_keys(int32_t n, int64_t E, const int32_t* __restrict__ u,
+__global__ void k_make_keys(int32_t n, int cb, int64_t E, const int32_t* __restrict__ u,
                             const int32_t* __restrict__ v, const int32_t* __restrict__ w,
                             int drop_self, unsigned long long* __restrict__ keys,
                             int32_t* __restrict__ vals, int32_t* __restrict__ err) {
@@ -72,76 +139,93 @@ __global__ void k_make_keys(int32_t n, int64_t E, const int32_t* __restrict__ u,
     bool skip = bad || (drop_self && a == b);
     unsigned long long ra = skip ? (unsigned long long)n : (unsigned long long)a;
     unsigned long long rb = skip ? (unsigned long long)n : (unsigned long long)b;
-    keys[2 * e] = (ra << 32) | (unsigned)(skip ? 0 : b);
-    keys[2 * e + 1] = (rb << 32) | (unsigned)(skip ? 0 : a);
-    vals[2 * e] = w[e];
-    vals[2 * e + 1] = w[e];
+    const int32_t x = w[e];
+    reinterpret_cast<ulonglong2*>(keys)[e] =
+        make_ulonglong2((ra << cb) | (unsigned)(skip ? 0 : b), (rb << cb) | (unsigned)(skip ? 0 : a));
+    reinterpret_cast<int2*>(vals)[e] = make_int2(x, x);
   }
 }
 
 // rowptr[r] = first sorted entry whose row >= r; entries with row == n are past the end.
-__global__ void k_rowptr(int32_t n, int64_t N, const unsigned long long* __restrict__ keys,
+__global__ void k_rowptr(int32_t n, int cb, int64_t N, const unsigned long long* __restrict__ keys,
                          int64_t* __restrict__ rowptr) {
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k <= N;
        k += (int64_t)gridDim.x * blockDim.x) {
-    int64_t rp = k == 0 ? -1 : (int64_t)(keys[k - 1] >> 32);
-    int64_t rc = k == N ? n : (int64_t)(keys[k] >> 32);
+    int64_t rp = k == 0 ? -1 : (int64_t)(keys[k - 1] >> cb);
+    int64_t rc = k == N ? n : (int64_t)(keys[k] >> cb);
     if (rp > n) rp = n;
     if (rc > n) rc = n;
     for (int64_t r = rp + 1; r <= rc; r++) rowptr[r] = k;
   }
 }
 
-__global__ void k_pack_adj(int64_t N, const unsigned long long* __restrict__ keys,
+// The kernels over entries run over all sorted keys and leave out those of row
+// n: how many there are is not known on the host yet.
+__global__ void k_pack_adj(int32_t n, int cb, int64_t N2, const unsigned long long* __restrict__ keys,
                            const int32_t* __restrict__ vals, int2* __restrict__ adj) {
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < N;
-       k += (int64_t)gridDim.x * blockDim.x)
-    adj[k] = make_int2((int32_t)(keys[k] & 0xffffffffu), vals[k]);
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < N2;
+       k += (int64_t)gridDim.x * blockDim.x) {
+    const unsigned long long key = keys[k];
+    if ((int64_t)(key >> cb) < n) adj[k] = make_int2((int32_t)(key & ((1ull << cb) - 1)), vals[k]);
+  }
 }
 
 // Per-row sum |w|: bounds |contribution| and decides the 32-bit key path
 // (out[0]); out[1] != 0 when some weight is negative; out[2] = max |w| (the
-// WSwap matrix holds 16-bit weights when it fits).
-__global__ void k_max_wdeg(int32_t n, const int64_t* __restrict__ rowptr,
-                           const int2* __restrict__ adj, unsigned long long* __restrict__ out,
-                           int2* __restrict__ wrange) {
-  for (int32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-    unsigned long long s = 0, mx = 0;
-    bool neg = false;
+// WSwap matrix holds 16-bit weights when it fits); the range of each row's
+// weights (the candidate pass leaves rows out by it).  A warp per row, one
+// atomic per block and result.
+__global__ void __launch_bounds__(kTPB)
+k_max_wdeg(int32_t n, const int64_t* __restrict__ rowptr, const int2* __restrict__ adj,
+           unsigned long long* __restrict__ out, int2* __restrict__ wrange) {
+  __shared__ unsigned long long s_sum, s_abs;
+  __shared__ int s_neg;
+  if (threadIdx.x == 0) { s_sum = 0; s_abs = 0; s_neg = 0; }
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  unsigned long long best = 0;
+  int32_t lo = 0, hi = 0;  // of all the warp's rows
+  for (int32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += (gridDim.x * blockDim.x) >> 5) {
+    unsigned long long sum = 0;
     int2 wr = make_int2(0, 0);  // of the row's weights and 0
-    for (int64_t k = rowptr[r]; k < rowptr[r + 1]; k++) {
-      int32_t x = adj[k].y;
-      const unsigned long long a = (unsigned long long)(x < 0 ? -(long long)x : (long long)x);
-      s += a;
-      mx = a > mx ? a : mx;
-      neg |= x < 0;
-      wr.x = x < wr.x ? x : wr.x;
-      wr.y = x > wr.y ? x : wr.y;
+    for (int64_t k = rowptr[r] + lane; k < rowptr[r + 1]; k += 32) {
+      const int32_t x = adj[k].y;
+      sum += (unsigned long long)(x < 0 ? -(long long)x : (long long)x);
+      wr.x = min(wr.x, x);
+      wr.y = max(wr.y, x);
     }
-    wrange[r] = wr;
-    atomicMax(out, s);
-    if (neg) atomicMax(out + 1, 1ull);
-    if (mx) atomicMax(out + 2, mx);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      wr.x = min(wr.x, __shfl_xor_sync(0xffffffffu, wr.x, o));
+      wr.y = max(wr.y, __shfl_xor_sync(0xffffffffu, wr.y, o));
+    }
+    if (lane == 0) wrange[r] = wr;
+    best = sum > best ? sum : best;
+    lo = min(lo, wr.x);
+    hi = max(hi, wr.y);
+  }
+  if (lane == 0) {
+    const unsigned long long a = (unsigned long long)(-(long long)lo), b = (unsigned long long)hi;
+    atomicMax(&s_sum, best);
+    atomicMax(&s_abs, a > b ? a : b);
+    if (lo < 0) atomicOr(&s_neg, 1);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (s_sum) atomicMax(out, s_sum);
+    if (s_neg) atomicMax(out + 1, 1ull);
+    if (s_abs) atomicMax(out + 2, s_abs);
   }
 }
 
-__device__ __forceinline__ int32_t row_of(const int64_t* rowptr, int32_t n, int64_t k) {
-  int32_t lo = 0, hi = n - 1;  // last row r with rowptr[r] <= k
-  while (lo < hi) {
-    int32_t mid = (lo + hi + 1) >> 1;
-    if (rowptr[mid] <= k) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
-__global__ void k_fill_bits(int32_t n, int64_t N, const int64_t* __restrict__ rowptr,
-                            const int2* __restrict__ adj, int64_t wpr,
+__global__ void k_fill_bits(int32_t n, int cb, int64_t N2, const unsigned long long* __restrict__ keys, int64_t wpr,
                             unsigned long long* __restrict__ bits) {
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < N;
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < N2;
        k += (int64_t)gridDim.x * blockDim.x) {
-    int32_t r = row_of(rowptr, n, k);
-    int32_t c = adj[k].x;
-    atomicOr(&bits[r * wpr + (c >> 6)], 1ull << (c & 63));
+    const int64_t r = (int64_t)(keys[k] >> cb);
+    const int32_t c = (int32_t)(keys[k] & ((1ull << cb) - 1));
+    if (r < n) atomicOr(&bits[r * wpr + (c >> 6)], 1ull << (c & 63));
   }
 }
 
@@ -151,22 +235,14 @@ __global__ void k_hash_caps(int32_t n, const int64_t* __restrict__ rowptr, int64
   if (blockIdx.x == 0 && threadIdx.x == 0) caps[n] = 0;
 }
 
-__global__ void k_hash_clear(int64_t slots, int32_t* __restrict__ keys, int32_t* __restrict__ vals) {
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < slots;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    keys[k] = kHashEmpty;
-    vals[k] = 0;
-  }
-}
-
 // Inserts the first entry of every (row, neighbour) pair with linear probing.
-__global__ void k_hash_insert(int32_t n, int64_t N, const int64_t* __restrict__ rowptr,
-                              const int2* __restrict__ adj, const int64_t* __restrict__ hoff,
+__global__ void k_hash_insert(int cb, int64_t N, const unsigned long long* __restrict__ sorted,
+                              const int64_t* __restrict__ rowptr, const int2* __restrict__ adj, const int64_t* __restrict__ hoff,
                               int32_t* __restrict__ keys, int32_t* __restrict__ vals,
                               int32_t* __restrict__ err) {
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < N;
        k += (int64_t)gridDim.x * blockDim.x) {
-    int32_t r = row_of(rowptr, n, k);
+    const int64_t r = (int64_t)(sorted[k] >> cb);
     int2 e = adj[k];
     if (k > rowptr[r] && adj[k - 1].x == e.x) continue;  // duplicate pair: first wins
     const int64_t base = hoff[r];
@@ -191,11 +267,14 @@ __global__ void k_hash_insert(int32_t n, int64_t N, const int64_t* __restrict__ 
 
 // rev[k] for entry k = (y -> z): the entry (z -> y) in row z with the same
 // duplicate rank (a self-loop's entries map to themselves).
-__global__ void k_reverse_index(int32_t n, int64_t N, const int64_t* __restrict__ rowptr,
-                                const int2* __restrict__ adj, int64_t* __restrict__ rev) {
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < N;
+__global__ void k_reverse_index(int32_t n, int cb, int64_t N2, const unsigned long long* __restrict__ keys,
+                                const int64_t* __restrict__ rowptr, const int2* __restrict__ adj,
+                                int64_t* __restrict__ rev) {
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < N2;
        k += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t y = row_of(rowptr, n, k);
+    const int64_t row = (int64_t)(keys[k] >> cb);
+    if (row >= n) continue;
+    const int32_t y = (int32_t)row;
     const int32_t z = adj[k].x;
     auto lower = [&](int32_t row, int32_t key) {
       int64_t lo = rowptr[row], len = rowptr[row + 1] - lo;
@@ -279,133 +358,148 @@ __global__ void k_lookup(DevGraph g, int64_t count, const int32_t* __restrict__ 
 }
 
 // ------------------------------------------------------------- build
-static ts_status build_graph(ts_graph* G, int64_t E, const int32_t* d_u, const int32_t* d_v,
-                             const int32_t* d_w) {
+// Builds from device arrays, or from host arrays (copied first).  All
+// temporaries are one allocation (pooled) and so are the graph's arrays (the
+// hash tables, whose size needs the degrees, another): an allocation or a free
+// synchronises and takes 50 us to milliseconds, and a build had 12 to 20 of
+// each.  One host round trip, two for Hash.  Conflict graph, n = 100,000, 3.4M
+// edges, from host arrays: Hash 11.2 -> 5.3 ms (2.3 of them the copies), CSR
+// 8.7 -> 5.2; a million lookups 3.3 -> 1.1 ms.
+static ts_status build_graph(ts_graph* G, int64_t E, const int32_t* u, const int32_t* v, const int32_t* w,
+                             bool on_host) {
   cudaStream_t st = G->stream;
   const int32_t n = G->n;
   const int64_t N2 = 2 * E;
-  DevBuf keys, keys_alt, vals, vals_alt, err, tmp, cnt;
+  const bool hash = G->kind == TS_STRUCT_HASH;
+  const bool bitset = G->kind == TS_STRUCT_CSR_BITSET || G->kind == TS_STRUCT_CSR_BITSET_BB;
   TS_CUDA(cudaSetDevice(G->device));
-  ts_status s;
-  if ((s = keys.alloc(sizeof(unsigned long long) * N2, "alloc keys")) != TS_OK) return s;
-  if ((s = keys_alt.alloc(sizeof(unsigned long long) * N2, "alloc keys")) != TS_OK) return s;
-  if ((s = vals.alloc(sizeof(int32_t) * N2, "alloc vals")) != TS_OK) return s;
-  if ((s = vals_alt.alloc(sizeof(int32_t) * N2, "alloc vals")) != TS_OK) return s;
-  if ((s = err.alloc(sizeof(int32_t) * 2, "alloc err")) != TS_OK) return s;
-  if ((s = cnt.alloc(3 * sizeof(unsigned long long), "alloc cnt")) != TS_OK) return s;
-  TS_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int32_t) * 2, st));
-  if (E > 0) {
-    k_make_keys<<<blocks_for(E), kTPB, 0, st>>>(n, E, d_u, d_v, d_w, G->drop_self_loops,
-                                                keys.as<unsigned long long>(), vals.as<int32_t>(),
-                                                err.as<int32_t>());
-    TS_CUDA(cudaGetLastError());
-  }
-  int row_bits = 1;
+  int row_bits = 1, cb = 1;
   while ((1LL << row_bits) <= (int64_t)n) row_bits++;
+  while ((1LL << cb) < (int64_t)n) cb++;
+  ts_status s;
+  DevParts temp;
+  DevPart hu, hv, hw, keys, keys_alt, vals, vals_alt, sum, tmp, caps;
+  const size_t eb = sizeof(int32_t) * (size_t)E;
+  if (on_host) {
+    temp.add(hu, eb);
+    temp.add(hv, eb);
+    temp.add(hw, eb);
+  }
+  temp.add(keys, sizeof(unsigned long long) * N2);
+  temp.add(keys_alt, sizeof(unsigned long long) * N2);
+  temp.add(vals, sizeof(int32_t) * N2);
+  temp.add(vals_alt, sizeof(int32_t) * N2);
+  // sum: wdeg results (3 words), then the error word
+  temp.add(sum, 4 * sizeof(unsigned long long));
+  if (hash) temp.add(caps, sizeof(int64_t) * (n + 1));
+  size_t sort_bytes = 0, scan_bytes = 0;
+  {
+    cub::DoubleBuffer<unsigned long long> dk;
+    cub::DoubleBuffer<int32_t> dv;
+    if (N2 > 0) TS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, dk, dv, N2, 0, cb + row_bits, st));
+    int64_t* none = nullptr;
+    if (hash) TS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, none, none, n + 1, st));
+  }
+  temp.add(tmp, sort_bytes > scan_bytes ? sort_bytes : scan_bytes);
+  if ((s = temp.alloc_temp("alloc build temporaries", st)) != TS_OK) return s;
+
+  G->mem.add(G->rowptr, sizeof(int64_t) * (n + 1));
+  // Two spare entries: the sweep bulk-copies rows from an even entry to an
+  // even end (16-byte aligned), which can reach one entry past the last row.
+  G->mem.add(G->adj, sizeof(int2) * (N2 + 2));
+  G->mem.add(G->wrange, sizeof(int2) * (size_t)n);
+  if (bitset) {
+    const int64_t words = ((int64_t)n + 63) / 64;
+    G->wpr = (words + 1) & ~1LL;  // even: every row starts on a 16 B boundary
+    G->mem.add(G->bits, sizeof(uint64_t) * (size_t)n * (size_t)G->wpr);
+  }
+  if (hash) G->mem.add(G->hoff, sizeof(int64_t) * (n + 1));
+  if (G->kind == TS_STRUCT_CSR) G->mem.add(G->rev, sizeof(int64_t) * (size_t)(N2 > 0 ? N2 : 1));
+  if ((s = G->mem.alloc("alloc graph")) != TS_OK) return s;
+
+  auto* d_sum = sum.as<unsigned long long>();
+  auto* d_err = reinterpret_cast<int32_t*>(d_sum + 3);
+  TS_CUDA(cudaMemsetAsync(d_sum, 0, 4 * sizeof(unsigned long long), st));
+  if (on_host && E > 0) {
+    TS_CUDA(cudaMemcpyAsync(hu.p, u, eb, cudaMemcpyHostToDevice, st));
+    TS_CUDA(cudaMemcpyAsync(hv.p, v, eb, cudaMemcpyHostToDevice, st));
+    TS_CUDA(cudaMemcpyAsync(hw.p, w, eb, cudaMemcpyHostToDevice, st));
+    u = hu.as<int32_t>();
+    v = hv.as<int32_t>();
+    w = hw.as<int32_t>();
+  }
   cub::DoubleBuffer<unsigned long long> dk(keys.as<unsigned long long>(), keys_alt.as<unsigned long long>());
   cub::DoubleBuffer<int32_t> dv(vals.as<int32_t>(), vals_alt.as<int32_t>());
-  if (N2 > 0) {
-    size_t tbytes = 0;
-    TS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tbytes, dk, dv, N2, 0, 32 + row_bits, st));
-    if ((s = tmp.alloc(tbytes, "alloc sort temp")) != TS_OK) return s;
-    TS_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tbytes, dk, dv, N2, 0, 32 + row_bits, st));
+  if (E > 0) {
+    k_make_keys<<<blocks_for(E), kTPB, 0, st>>>(n, cb, E, u, v, w, G->drop_self_loops, keys.as<unsigned long long>(),
+                                                vals.as<int32_t>(), d_err);
+    TS_CUDA(cudaGetLastError());
+    TS_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, sort_bytes, dk, dv, N2, 0, cb + row_bits, st));
   }
-  if ((s = G->rowptr.alloc(sizeof(int64_t) * (n + 1), "alloc rowptr")) != TS_OK) return s;
-  k_rowptr<<<blocks_for(N2 + 1), kTPB, 0, st>>>(n, N2, dk.Current(), G->rowptr.as<int64_t>());
+  k_rowptr<<<blocks_for(N2 + 1), kTPB, 0, st>>>(n, cb, N2, dk.Current(), G->rowptr.as<int64_t>());
   TS_CUDA(cudaGetLastError());
-  G->h_rowptr.assign(n + 1, 0);
-  TS_CUDA(cudaMemcpyAsync(G->h_rowptr.data(), G->rowptr.p, sizeof(int64_t) * (n + 1),
-                          cudaMemcpyDeviceToHost, st));
-  int32_t h_err[2] = {0, 0};
-  TS_CUDA(cudaMemcpyAsync(h_err, err.p, sizeof(int32_t) * 2, cudaMemcpyDeviceToHost, st));
+  if (E > 0) {
+    k_pack_adj<<<blocks_for(N2), kTPB, 0, st>>>(n, cb, N2, dk.Current(), dv.Current(), G->adj.as<int2>());
+    TS_CUDA(cudaGetLastError());
+  }
+  k_max_wdeg<<<blocks_for((int64_t)n * 32), kTPB, 0, st>>>(n, G->rowptr.as<int64_t>(), G->adj.as<int2>(), d_sum,
+                                                            G->wrange.as<int2>());
+  TS_CUDA(cudaGetLastError());
+  if (bitset) {
+    TS_CUDA(cudaMemsetAsync(G->bits.p, 0, G->bits.bytes, st));
+    if (E > 0) {
+      k_fill_bits<<<blocks_for(N2), kTPB, 0, st>>>(n, cb, N2, dk.Current(), G->wpr, G->bits.as<unsigned long long>());
+      TS_CUDA(cudaGetLastError());
+    }
+  }
+  if (G->kind == TS_STRUCT_CSR && E > 0) {
+    k_reverse_index<<<blocks_for(N2), kTPB, 0, st>>>(n, cb, N2, dk.Current(), G->rowptr.as<int64_t>(),
+                                                     G->adj.as<int2>(), G->rev.as<int64_t>());
+    TS_CUDA(cudaGetLastError());
+  }
+  int64_t slots = 0;
+  if (hash) {
+    k_hash_caps<<<blocks_for(n), kTPB, 0, st>>>(n, G->rowptr.as<int64_t>(), caps.as<int64_t>());
+    TS_CUDA(cudaGetLastError());
+    TS_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, scan_bytes, caps.as<int64_t>(), G->hoff.as<int64_t>(), n + 1, st));
+    TS_CUDA(cudaMemcpyAsync(&slots, G->hoff.as<int64_t>() + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  }
+  G->h_rowptr.resize(n + 1);
+  unsigned long long got[4] = {0, 0, 0, 0};
+  TS_CUDA(cudaMemcpyAsync(G->h_rowptr.data(), G->rowptr.p, sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToHost, st));
+  TS_CUDA(cudaMemcpyAsync(got, d_sum, sizeof(got), cudaMemcpyDeviceToHost, st));
   TS_CUDA(cudaStreamSynchronize(st));
-  if (h_err[0] & E_BAD_EDGE) {
+  if ((int32_t)got[3] & E_BAD_EDGE) {
     set_error("ts_graph_create: edge endpoint outside [0, n)");
     return TS_ERR_INVALID_ARG;
   }
   const int64_t N = G->h_rowptr[n];
   G->entries = N;
   G->num_edges = N / 2;
-  // Two spare entries: the sweep bulk-copies rows from an even entry to an
-  // even end (16-byte aligned), which can reach one entry past the last row.
-  if ((s = G->adj.alloc(sizeof(int2) * (N + 2), "alloc adj")) != TS_OK) return s;
-  if (N > 0) {
-    k_pack_adj<<<blocks_for(N), kTPB, 0, st>>>(N, dk.Current(), dv.Current(), G->adj.as<int2>());
-    TS_CUDA(cudaGetLastError());
-  }
-  keys.release();
-  keys_alt.release();
-  vals.release();
-  vals_alt.release();
-  tmp.release();
-  TS_CUDA(cudaMemsetAsync(cnt.p, 0, 3 * sizeof(unsigned long long), st));
-  if ((s = G->wrange.alloc(sizeof(int2) * (size_t)(n > 0 ? n : 1), "alloc row weight ranges")) != TS_OK) return s;
-  if (n > 0) {
-    k_max_wdeg<<<blocks_for(n), kTPB, 0, st>>>(n, G->rowptr.as<int64_t>(), G->adj.as<int2>(),
-                                               cnt.as<unsigned long long>(), G->wrange.as<int2>());
-    TS_CUDA(cudaGetLastError());
-  }
-  unsigned long long mw[3] = {0, 0, 0};
-  TS_CUDA(cudaMemcpyAsync(mw, cnt.p, sizeof(mw), cudaMemcpyDeviceToHost, st));
-
-  if (G->kind == TS_STRUCT_CSR_BITSET || G->kind == TS_STRUCT_CSR_BITSET_BB) {
-    int64_t words = ((int64_t)n + 63) / 64;
-    G->wpr = (words + 1) & ~1LL;  // even: every row starts on a 16 B boundary
-    size_t bytes = sizeof(uint64_t) * (size_t)n * (size_t)G->wpr;
-    if ((s = G->bits.alloc(bytes, "alloc bitset")) != TS_OK) return s;
-    TS_CUDA(cudaMemsetAsync(G->bits.p, 0, bytes, st));
-    if (N > 0) {
-      k_fill_bits<<<blocks_for(N), kTPB, 0, st>>>(n, N, G->rowptr.as<int64_t>(), G->adj.as<int2>(),
-                                                  G->wpr, G->bits.as<unsigned long long>());
-      TS_CUDA(cudaGetLastError());
-    }
-  }
-  if (G->kind == TS_STRUCT_HASH) {
-    if ((s = G->hoff.alloc(sizeof(int64_t) * (n + 1), "alloc hash offsets")) != TS_OK) return s;
-    DevBuf caps;
-    if ((s = caps.alloc(sizeof(int64_t) * (n + 1), "alloc hash caps")) != TS_OK) return s;
-    k_hash_caps<<<blocks_for(n), kTPB, 0, st>>>(n, G->rowptr.as<int64_t>(), caps.as<int64_t>());
-    TS_CUDA(cudaGetLastError());
-    size_t tbytes = 0;
-    TS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tbytes, caps.as<int64_t>(), G->hoff.as<int64_t>(),
-                                          n + 1, st));
-    if ((s = tmp.alloc(tbytes, "alloc scan temp")) != TS_OK) return s;
-    TS_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tbytes, caps.as<int64_t>(), G->hoff.as<int64_t>(),
-                                          n + 1, st));
-    int64_t slots = 0;
-    TS_CUDA(cudaMemcpyAsync(&slots, G->hoff.as<int64_t>() + n, sizeof(int64_t),
-                            cudaMemcpyDeviceToHost, st));
-    TS_CUDA(cudaStreamSynchronize(st));
+  G->max_wdeg = (int64_t)got[0];
+  G->neg_w = got[1] != 0;
+  G->max_abs_w = (int64_t)got[2];
+  if (hash) {
     G->hash_slots = slots;
-    if ((s = G->hkey.alloc(sizeof(int32_t) * slots, "alloc hash keys")) != TS_OK) return s;
-    if ((s = G->hval.alloc(sizeof(int32_t) * slots, "alloc hash weights")) != TS_OK) return s;
-    k_hash_clear<<<blocks_for(slots), kTPB, 0, st>>>(slots, G->hkey.as<int32_t>(), G->hval.as<int32_t>());
-    TS_CUDA(cudaGetLastError());
+    G->tables.add(G->hkey, sizeof(int32_t) * slots);
+    G->tables.add(G->hval, sizeof(int32_t) * slots);
+    if ((s = G->tables.alloc("alloc hash tables")) != TS_OK) return s;
+    TS_CUDA(cudaMemsetAsync(G->hkey.p, 0xff, G->hkey.bytes, st));  // kHashEmpty
+    TS_CUDA(cudaMemsetAsync(G->hval.p, 0, G->hval.bytes, st));
     if (N > 0) {
-      k_hash_insert<<<blocks_for(N), kTPB, 0, st>>>(n, N, G->rowptr.as<int64_t>(), G->adj.as<int2>(),
+      k_hash_insert<<<blocks_for(N), kTPB, 0, st>>>(cb, N, dk.Current(), G->rowptr.as<int64_t>(), G->adj.as<int2>(),
                                                     G->hoff.as<int64_t>(), G->hkey.as<int32_t>(),
-                                                    G->hval.as<int32_t>(), err.as<int32_t>());
+                                                    G->hval.as<int32_t>(), d_err);
       TS_CUDA(cudaGetLastError());
     }
-    TS_CUDA(cudaMemcpyAsync(h_err, err.p, sizeof(int32_t) * 2, cudaMemcpyDeviceToHost, st));
-  }
-  TS_CUDA(cudaStreamSynchronize(st));
-  if (h_err[0] & E_HASH_FULL) {
-    set_error("ts_graph_create: hash table overflow");
-    return TS_ERR_DEVICE;
-  }
-  if (G->kind == TS_STRUCT_CSR) {
-    if ((s = G->rev.alloc(sizeof(int64_t) * (size_t)(N > 0 ? N : 1), "alloc reverse index")) != TS_OK) return s;
-    if (N > 0) {
-      k_reverse_index<<<blocks_for(N), kTPB, 0, st>>>(n, N, G->rowptr.as<int64_t>(), G->adj.as<int2>(),
-                                                      G->rev.as<int64_t>());
-      TS_CUDA(cudaGetLastError());
-    }
+    int32_t err = 0;
+    TS_CUDA(cudaMemcpyAsync(&err, d_err, sizeof(err), cudaMemcpyDeviceToHost, st));
     TS_CUDA(cudaStreamSynchronize(st));
+    if (err & E_HASH_FULL) {
+      set_error("ts_graph_create: hash table overflow");
+      return TS_ERR_DEVICE;
+    }
   }
-  G->max_wdeg = (int64_t)mw[0];
-  G->neg_w = mw[1] != 0;
-  G->max_abs_w = (int64_t)mw[2];
   return TS_OK;
 }
 
@@ -413,18 +507,26 @@ static ts_status build_graph(ts_graph* G, int64_t E, const int32_t* d_u, const i
 
 using namespace tsb;
 
-static ts_status make_graph(int32_t n, int64_t E, const int32_t* d_u, const int32_t* d_v,
-                            const int32_t* d_w, int32_t kind, int32_t drop, void* stream,
-                            ts_graph** out) {
+static ts_status make_graph(int32_t n, int64_t E, const int32_t* u, const int32_t* v, const int32_t* w, int32_t kind,
+                            int32_t drop, void* stream, bool on_host, ts_graph** out) {
   if (!out) { set_error("ts_graph_create: out is NULL"); return TS_ERR_INVALID_ARG; }
   *out = nullptr;
+  if (on_host && (E < 0 || (E > 0 && (!u || !v || !w)))) {
+    set_error("ts_graph_create: bad edge arrays");
+    return TS_ERR_INVALID_ARG;
+  }
+  int ndev = 0;
+  if (on_host && (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)) {
+    cudaGetLastError();
+    set_error("no CUDA device visible");
+    return TS_ERR_NO_DEVICE;
+  }
   if (n < 2 || E < 0 || kind < 0 || kind >= TS_STRUCT_COUNT) {
     set_error("ts_graph_create: need n >= 2, num_edges >= 0 and a valid structure");
     return TS_ERR_INVALID_ARG;
   }
-  if (E > 0 && (!d_u || !d_v || !d_w)) { set_error("ts_graph_create: NULL edge array"); return TS_ERR_INVALID_ARG; }
-  int ndev = 0;
-  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
+  if (E > 0 && (!u || !v || !w)) { set_error("ts_graph_create: NULL edge array"); return TS_ERR_INVALID_ARG; }
+  if (!on_host && (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)) {
     cudaGetLastError();
     set_error("no CUDA device visible");
     return TS_ERR_NO_DEVICE;
@@ -435,8 +537,9 @@ static ts_status make_graph(int32_t n, int64_t E, const int32_t* d_u, const int3
   G->drop_self_loops = drop ? 1 : 0;
   G->stream = (cudaStream_t)stream;
   cudaGetDevice(&G->device);
-  ts_status s = build_graph(G, E, d_u, d_v, d_w);
+  ts_status s = build_graph(G, E, u, v, w, on_host);
   if (s != TS_OK) { delete G; return s; }
+  temp_users(G->device, 1);
   *out = G;
   return TS_OK;
 }
@@ -478,41 +581,14 @@ ts_status ts_graph_create_device(int32_t n, int64_t num_edges, const int32_t* d_
                                  const int32_t* d_w, int32_t kind, int32_t drop_self_loops,
                                  void* stream, ts_graph** out) {
   tsb::TraceRange tr_("ts_graph_create_device");
-  return make_graph(n, num_edges, d_u, d_v, d_w, kind, drop_self_loops, stream, out);
+  return make_graph(n, num_edges, d_u, d_v, d_w, kind, drop_self_loops, stream, false, out);
 }
 
 ts_status ts_graph_create(int32_t n, int64_t num_edges, const int32_t* u, const int32_t* v,
                           const int32_t* w, int32_t kind, int32_t drop_self_loops, void* stream,
                           ts_graph** out) {
   tsb::TraceRange tr_("ts_graph_create");
-  if (!out) { set_error("ts_graph_create: out is NULL"); return TS_ERR_INVALID_ARG; }
-  *out = nullptr;
-  if (num_edges < 0 || (num_edges > 0 && (!u || !v || !w))) {
-    set_error("ts_graph_create: bad edge arrays");
-    return TS_ERR_INVALID_ARG;
-  }
-  int ndev = 0;
-  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
-    cudaGetLastError();
-    set_error("no CUDA device visible");
-    return TS_ERR_NO_DEVICE;
-  }
-  cudaStream_t st = (cudaStream_t)stream;
-  DevBuf du, dv, dw;
-  ts_status s;
-  size_t b = sizeof(int32_t) * (size_t)num_edges;
-  if ((s = du.alloc(b, "alloc u")) != TS_OK) return s;
-  if ((s = dv.alloc(b, "alloc v")) != TS_OK) return s;
-  if ((s = dw.alloc(b, "alloc w")) != TS_OK) return s;
-  if (num_edges > 0) {
-    TS_CUDA(cudaMemcpyAsync(du.p, u, b, cudaMemcpyHostToDevice, st));
-    TS_CUDA(cudaMemcpyAsync(dv.p, v, b, cudaMemcpyHostToDevice, st));
-    TS_CUDA(cudaMemcpyAsync(dw.p, w, b, cudaMemcpyHostToDevice, st));
-  }
-  s = make_graph(n, num_edges, du.as<int32_t>(), dv.as<int32_t>(), dw.as<int32_t>(), kind,
-                 drop_self_loops, stream, out);
-  cudaStreamSynchronize(st);
-  return s;
+  return make_graph(n, num_edges, u, v, w, kind, drop_self_loops, stream, true, out);
 }
 
 ts_status ts_graph_info_get(const ts_graph* g, ts_graph_info* out) {
@@ -533,6 +609,7 @@ ts_status ts_graph_destroy(ts_graph* g) {
   if (!g) return TS_OK;
   cudaSetDevice(g->device);
   cudaStreamSynchronize(g->stream);
+  temp_users(g->device, -1);
   delete g;
   return TS_OK;
 }
@@ -561,12 +638,14 @@ ts_status ts_lookup_host(const ts_graph* g, int64_t count, const int32_t* u, con
   }
   if (count == 0) return TS_OK;
   TS_CUDA(cudaSetDevice(g->device));
-  DevBuf a, b, c;
+  DevParts mem;
+  DevPart a, b, c;
   size_t bytes = sizeof(int32_t) * (size_t)count;
   ts_status s;
-  if ((s = a.alloc(bytes, "alloc")) != TS_OK) return s;
-  if ((s = b.alloc(bytes, "alloc")) != TS_OK) return s;
-  if ((s = c.alloc(bytes, "alloc")) != TS_OK) return s;
+  mem.add(a, bytes);
+  mem.add(b, bytes);
+  mem.add(c, bytes);
+  if ((s = mem.alloc_temp("alloc lookup", g->stream)) != TS_OK) return s;
   TS_CUDA(cudaMemcpyAsync(a.p, u, bytes, cudaMemcpyHostToDevice, g->stream));
   TS_CUDA(cudaMemcpyAsync(b.p, v, bytes, cudaMemcpyHostToDevice, g->stream));
   s = ts_lookup(g, count, a.as<int32_t>(), b.as<int32_t>(), c.as<int32_t>());

@@ -6,6 +6,7 @@
 #include <memory>
 #include <random>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
@@ -37,6 +38,20 @@ ts_status cuda_fail(cudaError_t e, const char* what);
     if (e_ != cudaSuccess) return ::tsb::cuda_fail(e_, #call); \
   } while (0)
 
+// Temporaries of one call (build, lookup), taken from a memory pool of the
+// library's own per device and given back in stream order: an allocation of
+// hundreds of megabytes and its free cost milliseconds outside a pool.  The
+// pool keeps at most kTempKeep bytes between calls, kTempIdle once the last
+// graph is gone (emptying it costs a program that loads one small graph after
+// another 0.4 ms a graph), and nothing when an allocation of the library finds
+// no memory.
+constexpr size_t kTempKeep = 512u << 20;
+constexpr size_t kTempIdle = 32u << 20;
+cudaError_t temp_alloc(void** p, size_t bytes, cudaStream_t st);
+void temp_free(void* p, cudaStream_t st);
+void temp_trim();                 // current device: unused bytes back to the driver
+void temp_users(int device, int change);  // graphs alive on the device
+
 // Owning device buffer.
 struct DevBuf {
   void* p = nullptr;
@@ -54,6 +69,11 @@ struct DevBuf {
     release();
     if (nbytes == 0) nbytes = 16;
     cudaError_t e = cudaMalloc(&p, nbytes);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      temp_trim();
+      e = cudaMalloc(&p, nbytes);
+    }
     if (e != cudaSuccess) {
       p = nullptr;
       return cuda_fail(e, what);
@@ -62,6 +82,57 @@ struct DevBuf {
     return TS_OK;
   }
   template <class T> T* as() const { return static_cast<T*>(p); }
+};
+
+// Part of a device allocation that something else owns.
+struct DevPart {
+  void* p = nullptr;
+  size_t bytes = 0;
+  template <class T> T* as() const { return static_cast<T*>(p); }
+};
+// Parts of one allocation: sizes are registered first, then placed together
+// (every part starts on 256 bytes).
+struct DevParts {
+  DevBuf mem;
+  void* temp = nullptr;  // from the temporaries' pool, freed on `stream`
+  cudaStream_t stream = nullptr;
+  std::vector<std::pair<DevPart*, size_t>> parts;
+  DevParts() = default;
+  DevParts(const DevParts&) = delete;
+  DevParts& operator=(const DevParts&) = delete;
+  ~DevParts() {
+    if (temp) temp_free(temp, stream);
+  }
+  void add(DevPart& part, size_t bytes) {
+    part.bytes = bytes;
+    parts.emplace_back(&part, bytes);
+  }
+  ts_status alloc(const char* what) { return place(what, false); }
+  ts_status alloc_temp(const char* what, cudaStream_t st) {
+    stream = st;
+    return place(what, true);
+  }
+
+ private:
+  ts_status place(const char* what, bool pooled) {
+    auto pad = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    size_t total = 0;
+    for (auto& x : parts) total += pad(x.second);
+    if (pooled) {
+      const cudaError_t e = temp_alloc(&temp, total, stream);
+      if (e != cudaSuccess) return cuda_fail(e, what);
+    } else {
+      const ts_status rc = mem.alloc(total, what);
+      if (rc != TS_OK) return rc;
+    }
+    unsigned char* p = pooled ? static_cast<unsigned char*>(temp) : mem.as<unsigned char>();
+    for (auto& x : parts) {
+      x.first->p = p;
+      p += pad(x.second);
+    }
+    parts.clear();
+    return TS_OK;
+  }
 };
 
 }  // namespace tsb
@@ -79,7 +150,8 @@ struct ts_graph {
   int64_t max_abs_w = 0;  // largest |w| of an entry
   int64_t wpr = 0;
   int64_t hash_slots = 0;
-  tsb::DevBuf rowptr, adj, bits, hoff, hkey, hval, rev, wrange;
+  tsb::DevParts mem, tables;  // what is known before the sort; the hash tables
+  tsb::DevPart rowptr, adj, bits, hoff, hkey, hval, rev, wrange;
   // Host copy of the CSR row pointers/degrees (for footprint planning and the
   // solver's staging budgets); small: n+1 int64.
   std::vector<int64_t> h_rowptr;
