@@ -37,21 +37,21 @@ ts_status cuda_fail(cudaError_t e, const char* what) {
 
 namespace {
 constexpr int kMaxDevices = 64;
-struct TempPool {
+struct Pool {
   cudaMemPool_t pool = nullptr;
+  cudaStream_t stream = nullptr;  // allocations and frees for any stream
   bool tried = false;
   int users = 0;
 };
-std::mutex g_temp_mu;
-TempPool g_temp[kMaxDevices];
+std::mutex g_pool_mu;
+Pool g_pool[kMaxDevices];
 
-// The current device's pool; nullptr where there is none (temporaries are then
-// ordinary stream-ordered allocations of the device's default pool).
-cudaMemPool_t temp_pool() {
+// The current device's pool; without one (old driver) plain allocations are used.
+Pool* device_pool() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
-  std::lock_guard<std::mutex> lock(g_temp_mu);
-  TempPool& t = g_temp[dev];
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  Pool& t = g_pool[dev];
   if (!t.tried) {
     t.tried = true;
     cudaMemPoolProps props = {};
@@ -59,46 +59,71 @@ cudaMemPool_t temp_pool() {
     props.handleTypes = cudaMemHandleTypeNone;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
-    uint64_t keep = kTempKeep;
-    if (cudaMemPoolCreate(&t.pool, &props) != cudaSuccess) {
+    uint64_t keep = kPoolKeep;
+    if (cudaStreamCreateWithFlags(&t.stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaMemPoolCreate(&t.pool, &props) != cudaSuccess) {
       t.pool = nullptr;
       cudaGetLastError();
     } else {
       cudaMemPoolSetAttribute(t.pool, cudaMemPoolAttrReleaseThreshold, &keep);
     }
   }
-  return t.pool;
+  return t.pool ? &t : nullptr;
 }
 }  // namespace
 
-cudaError_t temp_alloc(void** p, size_t bytes, cudaStream_t st) {
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st) {
   *p = nullptr;
-  const cudaMemPool_t pool = temp_pool();
+  Pool* t = device_pool();
   for (int attempt = 0;; attempt++) {
-    const cudaError_t e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMallocAsync(p, bytes, st);
+    const cudaError_t e = t ? cudaMallocFromPoolAsync(p, bytes, t->pool, st) : cudaMallocAsync(p, bytes, st);
     if (e != cudaErrorMemoryAllocation || attempt) return e;
     cudaGetLastError();
-    temp_trim();
+    pool_trim();
   }
 }
-void temp_free(void* p, cudaStream_t st) {
+void pool_free(void* p, cudaStream_t st) {
   if (p) cudaFreeAsync(p, st);
 }
-void temp_trim() {
-  const cudaMemPool_t pool = temp_pool();
-  if (!pool) return;
-  cudaDeviceSynchronize();  // frees still queued on a stream
-  cudaMemPoolTrimTo(pool, 0);
-}
-void temp_users(int device, int change) {
-  bool last = false;
-  if (device < 0 || device >= kMaxDevices) return;
-  {
-    std::lock_guard<std::mutex> lock(g_temp_mu);
-    g_temp[device].users += change;
-    last = change < 0 && g_temp[device].users == 0 && g_temp[device].pool;
+cudaError_t pool_get(void** p, size_t bytes) {
+  Pool* t = device_pool();
+  if (bytes > kPoolBlock) {
+    for (int attempt = 0;; attempt++) {
+      const cudaError_t e = cudaMalloc(p, bytes);
+      if (e != cudaErrorMemoryAllocation || attempt) return e;
+      cudaGetLastError();
+      pool_trim();
+    }
   }
-  if (last) cudaMemPoolTrimTo(g_temp[device].pool, kTempIdle);
+  const cudaStream_t st = t ? t->stream : nullptr;
+  const cudaError_t e = pool_alloc(p, bytes, st);
+  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+void pool_put(void* p, size_t bytes) {
+  if (!p) return;
+  if (bytes > kPoolBlock) {
+    cudaFree(p);
+    return;
+  }
+  Pool* t = device_pool();
+  cudaDeviceSynchronize();
+  cudaFreeAsync(p, t ? t->stream : nullptr);
+}
+void pool_trim() {
+  Pool* t = device_pool();
+  if (!t) return;
+  cudaDeviceSynchronize();  // frees still queued on a stream
+  cudaMemPoolTrimTo(t->pool, 0);
+}
+void pool_users(int device, int change) {
+  if (device < 0 || device >= kMaxDevices) return;
+  cudaMemPool_t idle = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    g_pool[device].users += change;
+    if (change < 0 && g_pool[device].users == 0) idle = g_pool[device].pool;
+  }
+  if (idle) cudaMemPoolTrimTo(idle, kPoolIdle);
 }
 
 cudaError_t allow_dyn_smem(const void* fn, size_t smem) {
@@ -378,13 +403,8 @@ static ts_status build_graph(ts_graph* G, int64_t E, const int32_t* u, const int
   while ((1LL << cb) < (int64_t)n) cb++;
   ts_status s;
   DevParts temp;
-  DevPart hu, hv, hw, keys, keys_alt, vals, vals_alt, sum, tmp, caps;
+  DevPart keys, keys_alt, vals, vals_alt, sum, tmp, caps;
   const size_t eb = sizeof(int32_t) * (size_t)E;
-  if (on_host) {
-    temp.add(hu, eb);
-    temp.add(hv, eb);
-    temp.add(hw, eb);
-  }
   temp.add(keys, sizeof(unsigned long long) * N2);
   temp.add(keys_alt, sizeof(unsigned long long) * N2);
   temp.add(vals, sizeof(int32_t) * N2);
@@ -421,12 +441,15 @@ static ts_status build_graph(ts_graph* G, int64_t E, const int32_t* u, const int
   auto* d_err = reinterpret_cast<int32_t*>(d_sum + 3);
   TS_CUDA(cudaMemsetAsync(d_sum, 0, 4 * sizeof(unsigned long long), st));
   if (on_host && E > 0) {
-    TS_CUDA(cudaMemcpyAsync(hu.p, u, eb, cudaMemcpyHostToDevice, st));
-    TS_CUDA(cudaMemcpyAsync(hv.p, v, eb, cudaMemcpyHostToDevice, st));
-    TS_CUDA(cudaMemcpyAsync(hw.p, w, eb, cudaMemcpyHostToDevice, st));
-    u = hu.as<int32_t>();
-    v = hv.as<int32_t>();
-    w = hw.as<int32_t>();
+    // the sort's second buffers hold the edge arrays until the keys are made
+    int32_t* hu = keys_alt.as<int32_t>();  // 4 words per edge: u, v
+    int32_t* hw = vals_alt.as<int32_t>();
+    TS_CUDA(cudaMemcpyAsync(hu, u, eb, cudaMemcpyHostToDevice, st));
+    TS_CUDA(cudaMemcpyAsync(hu + E, v, eb, cudaMemcpyHostToDevice, st));
+    TS_CUDA(cudaMemcpyAsync(hw, w, eb, cudaMemcpyHostToDevice, st));
+    u = hu;
+    v = hu + E;
+    w = hw;
   }
   cub::DoubleBuffer<unsigned long long> dk(keys.as<unsigned long long>(), keys_alt.as<unsigned long long>());
   cub::DoubleBuffer<int32_t> dv(vals.as<int32_t>(), vals_alt.as<int32_t>());
@@ -539,7 +562,7 @@ static ts_status make_graph(int32_t n, int64_t E, const int32_t* u, const int32_
   cudaGetDevice(&G->device);
   ts_status s = build_graph(G, E, u, v, w, on_host);
   if (s != TS_OK) { delete G; return s; }
-  temp_users(G->device, 1);
+  pool_users(G->device, 1);
   *out = G;
   return TS_OK;
 }
@@ -609,8 +632,9 @@ ts_status ts_graph_destroy(ts_graph* g) {
   if (!g) return TS_OK;
   cudaSetDevice(g->device);
   cudaStreamSynchronize(g->stream);
-  temp_users(g->device, -1);
+  const int device = g->device;
   delete g;
+  pool_users(device, -1);
   return TS_OK;
 }
 

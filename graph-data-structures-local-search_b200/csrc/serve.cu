@@ -137,7 +137,7 @@ struct Req {
   ts_graph* g = nullptr;
   cudaStream_t stream = nullptr;   // plain: the graph's and solver's stream
   ts_solver* solver = nullptr;     // plain
-  std::unique_ptr<DevBuf> mem;     // packed: solver state, start, draws, result, best
+  std::unique_ptr<DevParts> mem;   // packed: solver state, start, draws, result, best
   std::vector<unsigned char> dev_solver;  // packed: DevSolver<KeyT> bytes
   DevGraph dg{};
   int32_t* d_init = nullptr;
@@ -251,7 +251,6 @@ ts_status build_packed(Req& r, int32_t kind) {
   const int64_t entries = r.g->entries;
   const int64_t events = r.p.problem == P_MAXBS ? r.p.max_iter / r.p.piter + 1 : 0;
   s.log_cap = r.p.max_iter + 1 + (r.p.problem == P_MAXBS ? (events + 1) * (int64_t)r.num_pert : 0);
-  auto pad = [](int64_t b) { return (b + 255) & ~255LL; };
   const int64_t sizes[] = {4 * m, 4 * ldc, 4 * m, 4 * ldc, 4 * (int64_t)n,
                            kind == S_CSR ? 4 * std::max<int64_t>(1, entries) : 0,
                            kind == S_WSWAP ? 4 * (int64_t)s.n_row_blocks * R * ldc : 0,
@@ -259,17 +258,14 @@ ts_status build_packed(Req& r, int32_t kind) {
                            8 * s.log_cap, 8 * std::max<int64_t>(1, events * r.num_pert),
                            4 * (int64_t)(r.p.problem == P_MDP ? m : n), (int64_t)sizeof(BatchResultDev),
                            4 * (int64_t)(r.p.problem == P_MDP ? m : n)};
-  int64_t total = 0;
-  for (int64_t x : sizes) total += pad(x);
-  r.mem.reset(new DevBuf);
-  ts_status rc = r.mem->alloc((size_t)total, "alloc served solve");
+  r.mem.reset(new DevParts);
+  DevPart part[15];
+  for (int i = 0; i < 15; i++)
+    if (sizes[i]) r.mem->add(part[i], (size_t)sizes[i]);
+  ts_status rc = r.mem->alloc("alloc served solve");
   if (rc != TS_OK) return rc;
-  unsigned char* b = r.mem->as<unsigned char>();
-  unsigned char* ptrs[15];
-  for (int i = 0; i < 15; i++) {
-    ptrs[i] = sizes[i] ? b : nullptr;
-    b += pad(sizes[i]);
-  }
+  void* ptrs[15];
+  for (int i = 0; i < 15; i++) ptrs[i] = part[i].p;
   s.sol_in = reinterpret_cast<int32_t*>(ptrs[0]);
   s.sol_out = reinterpret_cast<int32_t*>(ptrs[1]);
   s.tab_in = reinterpret_cast<int32_t*>(ptrs[2]);

@@ -481,7 +481,8 @@ struct ts_solver {
   int32_t num_pert = 1;
   int64_t log_cap = 0, trace_cap = 0;
   int64_t window_events = 0;
-  DevBuf sol_in, sol_out, vg_in, vg_out, tab_in, tab_out, pos, W, cpos, st, recs, movelog, trace, draws, work;
+  DevParts mem;  // all device arrays: one allocation
+  DevPart sol_in, sol_out, vg_in, vg_out, tab_in, tab_out, pos, W, cpos, st, recs, movelog, trace, draws, work;
   std::mt19937 rng;
   std::vector<long long> host_draws;  // every perturbation event drawn so far, k draws each
   int64_t events_drawn = 0;
@@ -587,27 +588,13 @@ ts_status prepare_draws(ts_solver* s, int64_t iters_ahead) {
   return TS_OK;
 }
 
-// Device scratch of the calls outside the iterations, kept with the solver: a
-// sum, the blocks' counts and a flag per vertex (init, result), or ids, stamps
-// and contributions (state, the largest).
-ts_status scratch(ts_solver* s, unsigned char** p) {
-  if (!s->work.p) {
-    const ts_status rc = s->work.alloc(16 * (size_t)s->n + 512, "alloc solver scratch");
-    if (rc != TS_OK) return rc;
-  }
-  *p = s->work.as<unsigned char>();
-  return TS_OK;
-}
-
 template <class KeyT>
 ts_status init_device(ts_solver* s, const std::vector<uint8_t>& inside) {
   const int32_t n = s->n, m = s->m;
   cudaStream_t st = s->g->stream;
   const int blocks = (n + kPlace - 1) / kPlace;
   const size_t counts = 256, flags = counts + 4 * (size_t)blocks;
-  unsigned char* w = nullptr;
-  ts_status rc;
-  if ((rc = scratch(s, &w)) != TS_OK) return rc;
+  unsigned char* w = s->work.as<unsigned char>();
   auto* acc = reinterpret_cast<unsigned long long*>(w);
   auto* count = reinterpret_cast<int32_t*>(w + counts);
   DevSolver<KeyT> d = s->dev<KeyT>();
@@ -642,9 +629,7 @@ ts_status init_device(ts_solver* s, const std::vector<uint8_t>& inside) {
 
 ts_status objective_of(ts_solver* s, const std::vector<uint8_t>& inside, long long* out) {
   cudaStream_t st = s->g->stream;
-  unsigned char* w = nullptr;
-  ts_status rc;
-  if ((rc = scratch(s, &w)) != TS_OK) return rc;
+  unsigned char* w = s->work.as<unsigned char>();
   auto* acc = reinterpret_cast<unsigned long long*>(w);
   TS_CUDA(cudaMemcpyAsync(w + 256, inside.data(), s->n, cudaMemcpyHostToDevice, st));
   TS_CUDA(cudaMemsetAsync(acc, 0, sizeof(unsigned long long), st));
@@ -775,28 +760,28 @@ ts_status ts_solver_create(ts_graph* g, const ts_params* p, ts_solver** out) {
   s->trace_cap = p->trace ? p->max_iter + pert_moves + 2 : 0;
   s->window_events = p->problem == TS_PROBLEM_MAXBS ? 64 : 1;
   const size_t kb = s->wide ? sizeof(long long) : sizeof(int32_t);
-  ts_status rc = TS_OK;
-  auto A = [&](DevBuf& b, size_t bytes, const char* what) {
-    if (rc == TS_OK) rc = b.alloc(bytes, what);
-  };
-  A(s->sol_in, sizeof(int32_t) * (size_t)m, "alloc sol_in");
-  A(s->sol_out, sizeof(int32_t) * (size_t)s->ldc, "alloc sol_out");
-  A(s->vg_in, kb * (size_t)m, "alloc vg_in");
-  A(s->vg_out, kb * (size_t)s->ldc, "alloc vg_out");
-  A(s->tab_in, sizeof(int32_t) * (size_t)m, "alloc tab_in");
-  A(s->tab_out, sizeof(int32_t) * (size_t)s->ldc, "alloc tab_out");
-  A(s->pos, sizeof(int32_t) * (size_t)n, "alloc pos");
-  A(s->st, sizeof(DevState), "alloc state");
-  A(s->recs, sizeof(CtaRec) * (size_t)s->grid, "alloc records");
-  A(s->movelog, sizeof(int2) * (size_t)s->log_cap, "alloc move log");
-  if (p->trace) A(s->trace, sizeof(TraceRec) * (size_t)s->trace_cap, "alloc trace");
-  A(s->draws, sizeof(long long) * (size_t)(s->window_events * s->num_pert), "alloc draws");
+  auto A = [&](DevPart& b, size_t bytes) { s->mem.add(b, bytes); };
+  A(s->sol_in, sizeof(int32_t) * (size_t)m);
+  A(s->sol_out, sizeof(int32_t) * (size_t)s->ldc);
+  A(s->vg_in, kb * (size_t)m);
+  A(s->vg_out, kb * (size_t)s->ldc);
+  A(s->tab_in, sizeof(int32_t) * (size_t)m);
+  A(s->tab_out, sizeof(int32_t) * (size_t)s->ldc);
+  A(s->pos, sizeof(int32_t) * (size_t)n);
+  A(s->st, sizeof(DevState));
+  A(s->recs, sizeof(CtaRec) * (size_t)s->grid);
+  A(s->movelog, sizeof(int2) * (size_t)s->log_cap);
+  if (p->trace) A(s->trace, sizeof(TraceRec) * (size_t)s->trace_cap);
+  A(s->draws, sizeof(long long) * (size_t)(s->window_events * s->num_pert));
   if (g->kind == S_WSWAP) {
     // Padded to whole row blocks so a tile never reads past the matrix.
     size_t rows = (size_t)s->n_row_blocks * s->R;
-    A(s->W, (s->w16 ? sizeof(int16_t) : sizeof(int32_t)) * rows * (size_t)s->ldc, "alloc WSwap matrix");
+    A(s->W, (s->w16 ? sizeof(int16_t) : sizeof(int32_t)) * rows * (size_t)s->ldc);
   }
-  if (g->kind == S_CSR) A(s->cpos, sizeof(int32_t) * (size_t)std::max<int64_t>(1, g->entries), "alloc cpos");
+  if (g->kind == S_CSR) A(s->cpos, sizeof(int32_t) * (size_t)std::max<int64_t>(1, g->entries));
+  // scratch of init, result and state: the last is the largest
+  A(s->work, 16 * (size_t)n + 512);
+  ts_status rc = s->mem.alloc("alloc solver");
   if (rc == TS_OK) {
     cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&s->h_st), sizeof(DevState));
     if (e != cudaSuccess) rc = cuda_fail(e, "cudaMallocHost state");
@@ -1077,9 +1062,7 @@ ts_status ts_solver_state(ts_solver* s, int32_t* sol, int32_t* pos, int32_t* tab
   cudaStream_t st = s->g->stream;
   const size_t n = (size_t)s->n;
   const size_t at_tab = 8 * n, at_sol = 12 * n;  // contributions first: 8-byte aligned
-  unsigned char* w = nullptr;
-  ts_status rc;
-  if ((rc = scratch(s, &w)) != TS_OK) return rc;
+  unsigned char* w = s->work.as<unsigned char>();
   auto* d_vg = reinterpret_cast<long long*>(w);
   auto* d_tab = reinterpret_cast<int32_t*>(w + at_tab);
   auto* d_sol = reinterpret_cast<int32_t*>(w + at_sol);

@@ -38,19 +38,27 @@ ts_status cuda_fail(cudaError_t e, const char* what);
     if (e_ != cudaSuccess) return ::tsb::cuda_fail(e_, #call); \
   } while (0)
 
-// Temporaries of one call (build, lookup), taken from a memory pool of the
-// library's own per device and given back in stream order: an allocation of
-// hundreds of megabytes and its free cost milliseconds outside a pool.  The
-// pool keeps at most kTempKeep bytes between calls, kTempIdle once the last
-// graph is gone (emptying it costs a program that loads one small graph after
-// another 0.4 ms a graph), and nothing when an allocation of the library finds
-// no memory.
-constexpr size_t kTempKeep = 512u << 20;
-constexpr size_t kTempIdle = 32u << 20;
-cudaError_t temp_alloc(void** p, size_t bytes, cudaStream_t st);
-void temp_free(void* p, cudaStream_t st);
-void temp_trim();                 // current device: unused bytes back to the driver
-void temp_users(int device, int change);  // graphs alive on the device
+// Device memory of graphs, solvers and calls comes from a memory pool of the
+// library's own per device: outside a pool an allocation or free of megabytes
+// costs 50 us to milliseconds and stalls every stream (ER n = 2,000: graph
+// 650 -> 150 us, its and its solver's end 450 -> 30 us).  The pool keeps at
+// most kPoolKeep unused bytes, kPoolIdle once the last graph is gone, and
+// nothing when an allocation of the library finds no memory.  Blocks above
+// kPoolBlock that outlive a call are plain allocations: the pool grows and
+// shrinks by many small mappings (a matrix of 1.8 GB: 10 ms and more, 0.5 ms
+// plain).
+//   pool_alloc/pool_free   in stream order (temporaries of one call);
+//   pool_get/pool_put      for any stream: ready on return; put waits for the
+//                          device, as a plain free does.
+constexpr size_t kPoolKeep = 512u << 20;
+constexpr size_t kPoolIdle = 256u << 20;
+constexpr size_t kPoolBlock = 64u << 20;
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st);
+void pool_free(void* p, cudaStream_t st);
+cudaError_t pool_get(void** p, size_t bytes);
+void pool_put(void* p, size_t bytes);
+void pool_trim();                         // current device: unused bytes back to the driver
+void pool_users(int device, int change);  // graphs alive on the device
 
 // Owning device buffer.
 struct DevBuf {
@@ -71,7 +79,7 @@ struct DevBuf {
     cudaError_t e = cudaMalloc(&p, nbytes);
     if (e == cudaErrorMemoryAllocation) {
       cudaGetLastError();
-      temp_trim();
+      pool_trim();
       e = cudaMalloc(&p, nbytes);
     }
     if (e != cudaSuccess) {
@@ -90,42 +98,46 @@ struct DevPart {
   size_t bytes = 0;
   template <class T> T* as() const { return static_cast<T*>(p); }
 };
-// Parts of one allocation: sizes are registered first, then placed together
-// (every part starts on 256 bytes).
+// Parts of one pool allocation: sizes are registered first, then placed
+// together (every part starts on 256 bytes).
 struct DevParts {
-  DevBuf mem;
-  void* temp = nullptr;  // from the temporaries' pool, freed on `stream`
+  void* mem = nullptr;
+  size_t bytes = 0;
+  bool ordered = false;  // freed in the order of `stream`
   cudaStream_t stream = nullptr;
   std::vector<std::pair<DevPart*, size_t>> parts;
   DevParts() = default;
   DevParts(const DevParts&) = delete;
   DevParts& operator=(const DevParts&) = delete;
   ~DevParts() {
-    if (temp) temp_free(temp, stream);
+    if (!mem) return;
+    if (ordered) pool_free(mem, stream);
+    else pool_put(mem, bytes);
   }
-  void add(DevPart& part, size_t bytes) {
-    part.bytes = bytes;
-    parts.emplace_back(&part, bytes);
+  void add(DevPart& part, size_t n) {
+    part.bytes = n;
+    parts.emplace_back(&part, n);
   }
-  ts_status alloc(const char* what) { return place(what, false); }
+  // For any stream, until the object goes.
+  ts_status alloc(const char* what) { return place(what); }
+  // For work on `st` alone.
   ts_status alloc_temp(const char* what, cudaStream_t st) {
+    ordered = true;
     stream = st;
-    return place(what, true);
+    return place(what);
   }
 
  private:
-  ts_status place(const char* what, bool pooled) {
-    auto pad = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    size_t total = 0;
-    for (auto& x : parts) total += pad(x.second);
-    if (pooled) {
-      const cudaError_t e = temp_alloc(&temp, total, stream);
-      if (e != cudaSuccess) return cuda_fail(e, what);
-    } else {
-      const ts_status rc = mem.alloc(total, what);
-      if (rc != TS_OK) return rc;
+  ts_status place(const char* what) {
+    auto pad = [](size_t b) { return b ? (b + 255) & ~(size_t)255 : (size_t)256; };
+    bytes = 0;
+    for (auto& x : parts) bytes += pad(x.second);
+    const cudaError_t e = ordered ? pool_alloc(&mem, bytes, stream) : pool_get(&mem, bytes);
+    if (e != cudaSuccess) {
+      mem = nullptr;
+      return cuda_fail(e, what);
     }
-    unsigned char* p = pooled ? static_cast<unsigned char*>(temp) : mem.as<unsigned char>();
+    unsigned char* p = static_cast<unsigned char*>(mem);
     for (auto& x : parts) {
       x.first->p = p;
       p += pad(x.second);
