@@ -389,8 +389,10 @@ ts_status ts_server_destroy(ts_server* s);
  * `stream` without synchronising, in the CUDA context current on the calling
  * thread (the device's primary context if none is).  The first call in each
  * context looks the scratch address up.  All calls share the scratch, so calls that overlap on the GPU
- * (other streams or host threads) race on it.  Cost: one binary search of a
- * global CSR row per pair, roughly P / 1e10 s for P = m*(n-m) pairs. */
+ * (other streams or host threads) race on it.  Cost: two
+ * launches; the rows and columns whose bounds can reach the best pair, or,
+ * where no pair is allowed and below 2^20 pairs, every pair with a binary search each (roughly
+ * P / 1e10 s for P = m*(n-m) pairs). */
 #define TS_NOALLOC_MAX_N 262144
 ts_status ts_best_swap_noalloc(int32_t problem, int32_t n, int32_t m, int64_t iter, int64_t cur,
                                int64_t best, const int64_t* d_rowptr, const int32_t* d_col,
