@@ -27,12 +27,20 @@ __device__ __forceinline__ long long block_sum(long long v, long long* sc) {
   return t;
 }
 
+// Lanes that share a row in the start and the result of a packed MDP solve.
+constexpr int kRowLanes = 8;
+
 // Start state of a solve in its slot, by one CTA: ascending ids per side
 // (initialSolution, GPU-MDP-CSR.cu:479-500), contributions and objective
 // (calculateVertexGain :502-519; computeGainsFromScratch /
 // computeFitnessFromScratch, GPU-MAXBS-CSR.cu:197-219), WSwap matrix
 // (calculateEdgeGain, GPU-MDP-WSwap.cu:607-626) and CSR neighbour positions.
-// The same values as the plain solver's init kernels.
+// The same values as the plain solver's init kernels.  MDP takes
+// eight lanes per selected row: the whole CTA on one row after another left
+// most threads idle on rows of 5-50 entries (n = 5,000, m = 625, degree 25,
+// start and result of a solve 0.56 -> 0.13 ms, with a WSwap matrix 1.1 -> 0.34).
+// Bisection's rows stay a thread each: there are n of them (0.18 ms; eight
+// lanes 0.41, a warp 0.76).
 template <int PROB, int ST, class KeyT>
 __device__ void slot_init(const DevGraph& g, const DevSolver<KeyT>& s, const int32_t* init,
                           long long max_iter, long long* sc, int32_t* s_cnt) {
@@ -50,6 +58,7 @@ __device__ void slot_init(const DevGraph& g, const DevSolver<KeyT>& s, const int
   s_cnt[tid] = cnt;
   __syncthreads();
   int32_t x = 0;
+#pragma unroll 8
   for (int t2 = 0; t2 < tid; t2++) x += s_cnt[t2];
   int32_t y = a0 - x;
   for (int32_t v = a0; v < a1; v++) {
@@ -59,14 +68,17 @@ __device__ void slot_init(const DevGraph& g, const DevSolver<KeyT>& s, const int
   for (int32_t j = s.delta + tid; j < s.ldc; j += T) s.sol_out[j] = 0;
   for (int32_t i = tid; i < m; i += T) { s.vg_in[i] = 0; s.tab_in[i] = 0; }
   for (int32_t j = tid; j < s.ldc; j += T) { s.vg_out[j] = 0; s.tab_out[j] = 0; }
-  if (ST == S_WSWAP)
-    for (long long q = tid; q < (long long)s.n_row_blocks * Rows<ST>::R * s.ldc; q += T) w_set(s, q, 0);
+  if (ST == S_WSWAP) {  // whole rows of ldc (a multiple of 4) elements
+    const long long words = (long long)s.n_row_blocks * Rows<ST>::R * s.ldc / (s.w16 ? 8 : 4);
+    for (long long q = tid; q < words; q += T) reinterpret_cast<int4*>(s.W)[q] = make_int4(0, 0, 0, 0);
+  }
   __syncthreads();
   long long acc = 0;
   if (PROB == P_MDP) {
-    for (int32_t i = 0; i < m; i++) {
+    for (int32_t i = tid / kRowLanes; i < m; i += T / kRowLanes) {
       const int32_t u = s.sol_in[i];
-      for (long long k = g.rowptr[u] + tid; k < g.rowptr[u + 1]; k += T) {
+#pragma unroll 4
+      for (long long k = g.rowptr[u] + tid % kRowLanes; k < g.rowptr[u + 1]; k += kRowLanes) {
         const int2 e = g.adj[k];
         const int32_t p = s.pos[e.x];
         atomic_add_key(vg_at(s, p), (KeyT)e.y);
@@ -93,10 +105,10 @@ __device__ void slot_init(const DevGraph& g, const DevSolver<KeyT>& s, const int
   if (ST == S_CSR)
     for (long long k = tid; k < g.entries; k += T) s.cpos[k] = s.pos[g.adj[k].x];
   if (ST == S_WSWAP) {
-    for (int32_t i = 0; i < m; i++) {
+    for (int32_t i = tid / kRowLanes; i < m; i += T / kRowLanes) {
       const int32_t u = s.sol_in[i];
       const long long k0 = g.rowptr[u];
-      for (long long k = k0 + tid; k < g.rowptr[u + 1]; k += T) {
+      for (long long k = k0 + tid % kRowLanes; k < g.rowptr[u + 1]; k += kRowLanes) {
         const int2 e = g.adj[k];
         if (k > k0 && g.adj[k - 1].x == e.x) continue;  // first entry of a duplicated pair
         const int32_t p = s.pos[e.x];
@@ -141,13 +153,15 @@ __device__ void slot_finish(const DevGraph& g, const DevSolver<KeyT>& s, BatchRe
   for (int32_t i = tid; i < s.m; i += T) s.pos[s.sol_in[i]] = 1;
   __syncthreads();
   long long acc = 0;
-  for (int32_t a = tid; a < s.n; a += T) {
+  constexpr int kLanes = PROB == P_MDP ? kRowLanes : 1;
+  for (int32_t x = tid / kLanes; x < (PROB == P_MDP ? s.m : s.n); x += T / kLanes) {
+    const int32_t a = PROB == P_MDP ? s.sol_in[x] : x;
     const int32_t fa = s.pos[a];
-    for (long long k = g.rowptr[a]; k < g.rowptr[a + 1]; k++) {
+    for (long long k = g.rowptr[a] + tid % kLanes; k < g.rowptr[a + 1]; k += kLanes) {
       const int2 e = g.adj[k];
       const int32_t fz = s.pos[e.x];
       if (PROB == P_MDP) {
-        if (fa && fz) acc += e.y;
+        if (fz) acc += e.y;
       } else if (e.x > a && fa != fz) {
         acc += e.y;
       }
