@@ -149,6 +149,13 @@ def algorithmic_bytes(kind: str, n: int, m: int, ldc: int, key_bytes: int, deg_i
     raise ValueError(kind)
 
 
+def candidate_bytes(n: int, key_bytes: int) -> int:
+    """Compulsory HBM bytes of a one-iteration launch of the candidate pass: it
+    reads every position's contribution, tabu stamp and vertex id and writes
+    them back (a launch of many iterations does so once)."""
+    return 2 * n * (key_bytes + 8)
+
+
 def profile_entry(workload: str, kind: str, grid: int):
     """Counters of one launch of this structure's iteration kernel on this
     workload, from an ncu capture (profiles/dram_traffic.json: DRAM bytes,
@@ -287,7 +294,10 @@ def run_ours(args):
 
     # per-structure compulsory bytes, from the state at the start of the timed region
     gi = graphs[kinds[0]].info()
-    solver_grid = {k: solvers[k].info().grid for k in kinds}
+    # default solvers run the candidate pass: a cluster launch and a guard
+    # launch per enqueue, in place of one sweep launch
+    cand = {k: solvers[k].info().cand_ctas for k in kinds}
+    solver_grid = {k: cand[k] or solvers[k].info().grid for k in kinds}
     w_bytes = max(1, solvers["wswap"].info().w_bytes) if "wswap" in kinds else 4
     words = (n + 63) // 64
     wpr = words + (words & 1)
@@ -305,7 +315,8 @@ def run_ours(args):
     cap_in = np.array([_hash_cap(int(d)) for d in deg_in], np.int64)
     ldc = (n - m + 3) // 4 * 4
     key_bytes = 4 if 4 * gi.max_weighted_degree < (1 << 30) else 8
-    bytes_per_iter = {k: algorithmic_bytes(k, n, m, ldc, key_bytes, deg_in, cap_in, wpr, w_bytes) for k in kinds}
+    bytes_per_iter = {k: candidate_bytes(n, key_bytes) if cand[k] else
+                      algorithmic_bytes(k, n, m, ldc, key_bytes, deg_in, cap_in, wpr, w_bytes) for k in kinds}
     del rowptr
 
     ev = {k: [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
@@ -350,7 +361,7 @@ def run_ours(args):
         avg_s = ms / 1e3 / args.steps
         per[k] = {"iters_per_s": 1.0 / avg_s, "swap_gains_per_s": P / avg_s, "ms_per_iter": ms / args.steps,
                   "bytes_per_iter": bytes_per_iter[k], "achieved_gbs": bytes_per_iter[k] / avg_s / 1e9,
-                  "grid": solver_grid[k]}
+                  "grid": solver_grid[k], "pass": "candidate" if cand[k] else "sweep"}
     t_max_ms, value = whole_job_value(tot_ms, ws, P * len(kinds) * args.steps, dev)
 
     peak, peak_src = measured_peaks()
@@ -358,7 +369,7 @@ def run_ours(args):
     achieved = per[dom]["achieved_gbs"]
     csum = clocks.summary()
     sm_mhz = csum["sm_mhz"] or csum["sm_max_mhz"] or 1965.0
-    prof = {k: profile_entry(args.workload, k, solver_grid[k]) for k in kinds}
+    prof = {k: None if cand[k] else profile_entry(args.workload, k, solver_grid[k]) for k in kinds}
     for k in kinds:
         pe = prof[k]
         if pe and pe.get("warp_inst"):
@@ -367,14 +378,15 @@ def run_ours(args):
             per[k]["l2_hit_rate_ncu"] = pe.get("l2_hit_pct")
             per[k]["threads_per_warp_inst_ncu"] = pe.get("threads_per_inst")
     traffic = prof[dom]["bytes"] if prof[dom] else None
-    roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                "frac": achieved / peak, "traffic": traffic, "kernel": f"iter_kernel[{dom}]",
+    roofline = {"bound": "latency" if cand[dom] else "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                "frac": achieved / peak, "traffic": traffic,
+                "kernel": f"{'cand' if cand[dom] else 'iter'}_kernel[{dom}]",
                 "peak_source": peak_src,
                 "int_issue_frac": per[dom].get("int_issue_frac"),
                 "note": "dominant kernel = slowest structure per iteration; int_issue_frac = its warp "
                         "instructions per launch (ncu capture of the same grid) / measured launch time / "
                         "(148 SMs x 4 schedulers x SM clock)"}
-    if "wswap" in per:  # the structure whose sweep is HBM-bound: the matrix streams once per iteration
+    if "wswap" in per and not cand["wswap"]:  # its sweep is HBM-bound: the matrix streams once per iteration
         roofline["hbm_bound_kernel"] = {"kernel": "iter_kernel[wswap]", "achieved": per["wswap"]["achieved_gbs"],
                                         "frac": per["wswap"]["achieved_gbs"] / peak}
 
@@ -383,6 +395,13 @@ def run_ours(args):
         graphs[k].close()
     del flush
     torch.cuda.empty_cache()
+    if rank == 0 and not args.no_extras and "wswap" in kinds and cand["wswap"]:
+        # the sweep that the candidate pass stands in for, pinned
+        w, _, _ = time_structures(T, torch, dev, stream, wl, problem, m, ["wswap"], iters=20, warmup=3,
+                                  flush_between=True, sweep=T.PASS_TILE)
+        gbs = algorithmic_bytes("wswap", n, m, ldc, key_bytes, deg_in, cap_in, wpr, w_bytes) * w["wswap"]["iters_per_s"] / 1e9
+        roofline["hbm_bound_kernel"] = {"kernel": "iter_kernel[wswap], pinned sweep", "achieved": gbs, "frac": gbs / peak,
+                                        "iters_per_s": w["wswap"]["iters_per_s"]}
 
     line = None
     if rank == 0:
@@ -398,6 +417,8 @@ def run_ours(args):
             "scaling": "weak", "vs_baseline": None, "dtype": "int32",
             "data": "synthetic (seeded conflict-style graph; MWIS-VR instances are not available offline)",
             "config": {"workload": wl["desc"], "n": n, "m": m, "pairs_per_iter": P, "structures": kinds,
+                       "pairs": "each iteration decides the best of all pairs; the candidate pass excludes pairs "
+                                "by bounds (evaluated one by one: --sweep tile or rows)",
                        "l2": "256 MiB buffer written between timed iterations (outside the events)",
                        "parallelism": f"replicas x{ws}" if ws > 1 else "single GPU"},
             "iters_per_s": len(kinds) * args.steps / (t_max_ms / 1e3),
@@ -410,7 +431,7 @@ def run_ours(args):
             "reference_cuda": ref_cuda,
             "batched": batched,
             "served": served,
-            "gpu_launches": len(kinds) * args.steps,
+            "gpu_launches": sum(2 if cand[k] else 1 for k in kinds) * args.steps,
             "clocks": csum,
             "wall_s_timed_region": wall,
         }
@@ -437,7 +458,7 @@ def gpu_head_start(torch, launches: int):
     torch.cuda._sleep(int(seconds * 2.0e9))
 
 
-def time_structures(T, torch, dev, stream, wl, problem, m, kinds, iters, warmup, flush_between, seed=1):
+def time_structures(T, torch, dev, stream, wl, problem, m, kinds, iters, warmup, flush_between, seed=1, sweep=0):
     """Plain solves of one workload, one structure at a time (built, started
     from the same seeded state, `warmup` untimed iterations, then `iters`
     timed ones).  flush_between: a 256 MiB buffer is written before every
@@ -452,7 +473,7 @@ def time_structures(T, torch, dev, stream, wl, problem, m, kinds, iters, warmup,
     for k in kinds:
         g = T.Graph(n, wl["u"], wl["v"], wl["w"], k, drop_self_loops=mdp, stream=stream.cuda_stream)
         s = T.Solver(g, problem, m=m if mdp else 0, max_iter=10**9, tenure_policy=T.TENURE_FIXED,
-                     tenure=wl["tenure"], piter=500, gamma=150, seed=seed)
+                     tenure=wl["tenure"], piter=500, gamma=150, seed=seed, sweep=sweep)
         try:
             s.init(None)
             assert s.prepare(warmup + iters) == warmup + iters
@@ -487,7 +508,7 @@ def time_structures(T, torch, dev, stream, wl, problem, m, kinds, iters, warmup,
             g.close()
         sec = ms / 1e3 / iters
         out[k] = {"iters_per_s": 1.0 / sec, "swap_gains_per_s": P / sec, "ms_per_iter": ms / iters,
-                  "grid": si.grid, "w_bytes": si.w_bytes, "_state": st}
+                  "grid": si.cand_ctas or si.grid, "cand_ctas": si.cand_ctas, "w_bytes": si.w_bytes, "_state": st}
         if len(each) > 1:
             out[k]["ms_first_last"] = [round(each[0], 4), round(each[-1], 4)]
     states = [out[k].pop("_state") for k in kinds]
@@ -522,7 +543,8 @@ def run_configs(T, torch, dev, stream, kinds):
     wpr = words + (words & 1)
     ldc = (n - m + 3) // 4 * 4
     for k in kinds:
-        b = algorithmic_bytes(k, n, m, ldc, 4, deg_in, cap_in, wpr, w_bytes=max(1, per[k]["w_bytes"]))
+        b = candidate_bytes(n, 4) if per[k]["cand_ctas"] else \
+            algorithmic_bytes(k, n, m, ldc, 4, deg_in, cap_in, wpr, w_bytes=max(1, per[k]["w_bytes"]))
         per[k]["bytes_per_iter"] = b
         per[k]["achieved_gbs"] = b * per[k]["iters_per_s"] / 1e9
         per[k]["hbm_frac"] = per[k]["achieved_gbs"] / peak

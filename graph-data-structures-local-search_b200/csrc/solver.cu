@@ -1147,6 +1147,7 @@ ts_status ts_solver_info_get(const ts_solver* s, ts_solver_info* out) {
   out->key_bytes = s->wide ? 8 : 4;
   out->w_bytes = s->g->kind == S_WSWAP ? (s->w16 ? 2 : 4) : 0;
   out->slices = s->n_slices;
+  out->cand_ctas = s->cand.cs;
   return TS_OK;
 }
 

@@ -3,7 +3,8 @@
 For every (problem, size bucket) it times short batches of a representative
 instance on each candidate lookup structure, cluster size (CTAs per solve)
 and pair sweep (the tile pass: 32 rows per tile, one structure query per
-column; or the per-row pass: a few rows per tile, one lookup per pair) and
+column; the per-row pass: a few rows per tile, one lookup per pair; or the
+library's default, the candidate pass, at the library's cluster size) and
 keeps the fastest, measured as swap pairs evaluated per second of device
 time.  Results do not depend on the choice -- every structure, cluster size
 and sweep gives the same trajectory -- so the table only decides speed.
@@ -31,7 +32,7 @@ class Choice:
 
 
 class Table:
-    """(problem, n) -> (structure, cluster size)."""
+    """(problem, n) -> (structure, cluster size; 0: the library's choice)."""
 
     def __init__(self, buckets=DEFAULT_BUCKETS):
         self.buckets = tuple(buckets)
@@ -109,17 +110,22 @@ def autotune(buckets=DEFAULT_BUCKETS, kinds=("csr", "wswap", "csr-bb", "hash"), 
                     for sw in sweeps:
                         if kind == "wswap" and sw == C.PASS_TILE:
                             continue  # the matrix has one sweep
+                        # the default pass keeps a solve's state in the cluster's
+                        # shared memory: the library sizes the cluster by the solve
+                        ctas = 0 if sw == C.PASS_AUTO else cs
+                        if ctas == 0 and cs != clusters[0]:
+                            continue
                         if time.perf_counter() - t_start > budget and best is not None:
                             break
                         try:
-                            rate = _trial(problem, n, kind, cs, jobs, iters, seed + b, sw)
+                            rate = _trial(problem, n, kind, ctas, jobs, iters, seed + b, sw)
                         except C.TsError as e:  # this shape does not fit the device: not a candidate
-                            table.trials.append({"problem": problem, "n": n, "structure": kind, "cluster": cs,
+                            table.trials.append({"problem": problem, "n": n, "structure": kind, "cluster": ctas,
                                                  "sweep": sw, "unavailable": str(e)})
                             continue
-                        table.trials.append({"problem": problem, "n": n, "structure": kind, "cluster": cs,
+                        table.trials.append({"problem": problem, "n": n, "structure": kind, "cluster": ctas,
                                              "sweep": sw, "pairs_per_s": rate})
                         if best is None or rate > best.pairs_per_s:
-                            best = Choice(kind, cs, rate, sw)
+                            best = Choice(kind, ctas, rate, sw)
             table.choice[(problem, b)] = best
     return table

@@ -105,7 +105,8 @@ typedef struct ts_solver_info {
   int32_t key_bytes;      /* 4: 32-bit pair keys and contributions, 8: 64-bit */
   int32_t w_bytes;        /* WSwap: bytes per matrix element (2 or 4); 0 otherwise */
   int32_t slices;         /* CTAs per tile (grid = row blocks x n_chunks x slices) */
-  int32_t reserved[7];
+  int32_t cand_ctas;      /* CTAs of the candidate pass's cluster; 0: sweeps only */
+  int32_t reserved[6];
 } ts_solver_info;
 
 typedef struct ts_params {
