@@ -48,7 +48,7 @@ struct BatchJobDev {
   int32_t orig;             // index in the caller's job array
   int32_t adj_mask;         // CSR: adjacent pairs masked out of the w-free sweep
   int32_t tile_rows, fast, fast_ecap;  // tile shape (tile_geometry)
-  int32_t cand_rpc, cand_cpc, cand_vpc, cand_fav;  // candidate pass (cand_persist); 0: tiles only
+  int32_t cand_rpc, cand_cpc, cand_vpc, cand_fav, cand_list;  // candidate pass (cand_persist); 0: tiles only
   uint32_t cand_inv[3];
   long long cand_plus, cand_pairs;
   const int32_t* init;      // MDP: m ids; MaxBS: part[n]
@@ -86,7 +86,7 @@ __device__ DevSolver<KeyT> slot_solver(const BatchJobDev& J, const SlotPool<KeyT
   s.fast = J.fast;
   s.fast_ecap = J.fast_ecap;
   s.n_slices = 1;
-  s.cand_rpc = J.cand_rpc; s.cand_cpc = J.cand_cpc; s.cand_vpc = J.cand_vpc;
+  s.cand_rpc = J.cand_rpc; s.cand_cpc = J.cand_cpc; s.cand_vpc = J.cand_vpc; s.cand_list = J.cand_list;
   for (int k = 0; k < 3; k++) s.cand_inv[k] = J.cand_inv[k];
   s.cand_fav = J.cand_fav;
   s.cand_plus = J.cand_plus; s.cand_pairs = J.cand_pairs;
@@ -276,6 +276,7 @@ ts_status plan_group(Group& G, std::vector<BatchJobDev>& table, int64_t budget_b
     J.cand_rpc = cp.cs ? cp.rpc : 0;
     J.cand_cpc = cp.cpc;
     J.cand_vpc = cp.vpc;
+    J.cand_list = cp.list;
     for (int k = 0; k < 3; k++) J.cand_inv[k] = cp.inv[k];
     J.cand_fav = cp.fav;
     J.cand_plus = cp.plus;

@@ -101,11 +101,23 @@ CandPlan cand_slices(const ts_graph* g, int32_t problem, int32_t m, bool wide, i
   p.rpc = ((m + cs - 1) / cs + 3) & ~3;
   p.cpc = ((delta + cs - 1) / cs + 3) & ~3;
   const int kb = wide ? 8 : 4;
-  // Positions by vertex go to shared memory where they fit.
+  // Lists for three quarters of the slice (sparse graphs of few distinct
+  // contributions have that many candidates) or what fits, then the positions
+  // by vertex where they fit too.
+  const bool edges = p.plus > 0;
+  const int32_t whole = p.rpc + p.cpc;
+  const size_t bare = cand_layout(g->n, p.rpc, p.cpc, kb, 0, edges, 0).total;
+  int64_t list = std::min<int64_t>(std::max<int64_t>(kCandList, (int64_t)whole * 3 / 4), whole);
+  if (bare < limit) list = std::min<int64_t>(list, (int64_t)(limit - bare) / 8);
+  p.list = (int32_t)(std::max<int64_t>(list, std::min<int32_t>(whole, kCandList)) + 3) & ~3;
+  if (p.list > whole) p.list = whole;
   const int32_t vpc = ((g->n + cs - 1) / cs + 3) & ~3;
-  const bool map = p.plus > 0;
-  p.vpc = cand_layout(g->n, p.rpc, p.cpc, kb, vpc, map).total <= limit ? vpc : 0;
-  p.smem = cand_layout(g->n, p.rpc, p.cpc, kb, p.vpc, map).total;
+  p.vpc = cand_layout(g->n, p.rpc, p.cpc, kb, vpc, edges, p.list).total <= limit ? vpc : 0;
+  p.smem = cand_layout(g->n, p.rpc, p.cpc, kb, p.vpc, edges, p.list).total;
+  if (p.smem > limit && p.list > kCandList) {  // rounding of the fit
+    p.list -= 4;
+    p.smem = cand_layout(g->n, p.rpc, p.cpc, kb, p.vpc, edges, p.list).total;
+  }
   p.threads = kCandTPB;
   // Divisions by a slice are a multiplication by ceil(2^32 / slice), exact
   // for up to 16 slices of fewer than 2^14.
@@ -145,10 +157,11 @@ CandPlan cand_plan(const ts_graph* g, int32_t problem, int32_t m, bool wide) {
   // no cluster barriers.  1 / 8 / 16 CTAs, us per iteration: MDP ER n = 2,000
   // 2.5 / 3.5 / 3.7; dense n = 2,000 7.8 / 8.6 / 10.4; bisection n = 5,000
   // 14.5 / 10.1 / 10.4, n = 30,011 16.8 / 10.6 / 10.3, n = 100,000 - / 16.5 /
-  // 13.9.
+  // 13.9; n = 18,000 of degree 5 (half of the vertices are candidates) - / 23 /
+  // 17, n = 1,000 of degree 5 16 / 9.5 / -, of degree 25 8.3 / 9.6 / -.
   const int n = g->n;
   const bool edges = problem == P_MAXBS || g->neg_w;
-  int cs = edges ? (n <= 4096 ? 1 : (n <= 32768 ? 8 : 16)) : (n <= 8192 ? 1 : (n <= 32768 ? 4 : 16));
+  int cs = edges ? (n <= 768 ? 1 : (n <= 12288 ? 8 : 16)) : (n <= 8192 ? 1 : (n <= 32768 ? 4 : 16));
   for (; cs <= kCandMaxCluster; cs *= 2) {
     CandPlan p = cand_slices(g, problem, m, wide, cs, kCandSmem);
     p.threads = n <= 1024 ? 256 : kCandTPB;

@@ -44,7 +44,7 @@ namespace tsb {
 
 constexpr int kCandTPB = 512;        // most threads per CTA
 constexpr int kCandMaxCluster = 16;
-constexpr int kCandList = 2048;      // entries of a CTA's candidate lists
+constexpr int kCandList = 2048;      // entries of a CTA's candidate lists, at least (or its whole slice)
 constexpr int kCandStage = 1024;     // candidate columns staged per round of N
 constexpr int kCandHeavy = 512;      // E: rows of more entries are walked by the whole CTA
 constexpr int kCandHeavyList = 64;
@@ -63,7 +63,8 @@ struct CandLayout {
 // Shared memory of one CTA: rpc rows and cpc columns (multiples of 4), a slice
 // of the positions by vertex (vpc > 0), lists, for E the candidates' bitmap
 // and a queue, and one area for the staged columns (N) or rows (E).
-__host__ __device__ inline CandLayout cand_layout(int32_t n, int32_t rpc, int32_t cpc, int kb, int32_t vpc, bool edges) {
+__host__ __device__ inline CandLayout cand_layout(int32_t n, int32_t rpc, int32_t cpc, int kb, int32_t vpc, bool edges,
+                                                      int32_t list) {
   CandLayout L;
   uint32_t off = 0;
   L.va = off; off += (uint32_t)kb * rpc;
@@ -74,7 +75,7 @@ __host__ __device__ inline CandLayout cand_layout(int32_t n, int32_t rpc, int32_
   L.ub = off; off += 4u * cpc;
   L.vpc = vpc;
   L.pv = off; off += 4u * (uint32_t)vpc;
-  L.rcap = L.ccap = rpc + cpc < kCandList ? rpc + cpc : kCandList;
+  L.rcap = L.ccap = list;
   L.rl = off; off += 4u * (uint32_t)L.rcap;
   L.cl = off; off += 4u * (uint32_t)L.ccap;
   L.map_bytes = edges ? 16u * (uint32_t)((n + 127) / 128) : 0u;
@@ -383,7 +384,7 @@ __device__ int cand_run(const DevGraph& g, const DevSolver<KeyT>& s, long long s
   const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = T >> 5;
   const int nb = (int)cl.num_blocks(), rank = (int)cl.block_rank();
   const int32_t m = s.m, delta = s.delta, rpc = s.cand_rpc, cpc = s.cand_cpc;
-  const CandLayout L = cand_layout(s.n, rpc, cpc, kKb, s.cand_vpc, s.cand_plus > 0);
+  const CandLayout L = cand_layout(s.n, rpc, cpc, kKb, s.cand_vpc, s.cand_plus > 0, s.cand_list);
   // one array each: the slice's rows, then (from rpc) its columns
   KeyT* val = reinterpret_cast<KeyT*>(smem + L.va);
   int32_t* stamp = reinterpret_cast<int32_t*>(smem + L.ta);

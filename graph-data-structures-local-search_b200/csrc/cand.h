@@ -13,6 +13,7 @@ struct CandPlan {
   int32_t rpc = 0, cpc = 0; // rows and columns per CTA (multiples of 4)
   int32_t vpc = 0;          // vertices per CTA of the position slice; 0: positions stay in HBM
   uint32_t inv[3] = {0, 0, 0};  // ceil(2^32 / slice): rows, columns, vertices
+  int32_t list = 0;         // entries of a CTA's candidate lists
   int32_t fav = 0;          // every c*w >= 0
   int64_t plus = 0;         // upper bound of c*w
   int64_t pairs = 0;        // candidate pairs per CTA before a sweep is cheaper

@@ -242,6 +242,7 @@ ts_status build_packed(Req& r, int32_t kind) {
   s.cand_rpc = cp.cs ? cp.rpc : 0;
   s.cand_cpc = cp.cpc;
   s.cand_vpc = cp.vpc;
+  s.cand_list = cp.list;
   for (int k = 0; k < 3; k++) s.cand_inv[k] = cp.inv[k];
   s.cand_fav = cp.fav;
   s.cand_plus = cp.plus;

@@ -515,7 +515,7 @@ struct ts_solver {
     s.fast_ecap = fast_ecap;
     s.n_slices = n_slices;
     s.w16 = w16;
-    s.cand_rpc = cand.rpc; s.cand_cpc = cand.cpc; s.cand_vpc = cand.vpc;
+    s.cand_rpc = cand.rpc; s.cand_cpc = cand.cpc; s.cand_vpc = cand.vpc; s.cand_list = cand.list;
     for (int k = 0; k < 3; k++) s.cand_inv[k] = cand.inv[k];
     s.cand_fav = cand.fav; s.cand_plus = cand.plus; s.cand_pairs = cand.pairs;
     s.P = P;

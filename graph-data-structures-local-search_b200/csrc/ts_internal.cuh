@@ -112,6 +112,7 @@ struct DevSolver {
   // of the positions by vertex (0: read from HBM), whether every c*w >= 0 (Max Bisection without negative weights) and the
   // upper bound of c*w over the graph's edges.
   int32_t cand_rpc, cand_cpc, cand_vpc, cand_fav;
+  int32_t cand_list;      // entries of a CTA's candidate lists (a multiple of 4)
   uint32_t cand_inv[3];   // ceil(2^32 / slice): rows, columns, vertices
   int32_t guard;          // this launch runs only while DevState::owed > 0
   int64_t cand_plus;
