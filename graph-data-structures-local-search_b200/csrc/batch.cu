@@ -8,8 +8,9 @@
 // Here solves are grouped by (problem, structure, key width, CTAs per solve)
 // and each group is ONE persistent launch.  A thread-block cluster of 1-8 CTAs
 // owns one slot of solver memory in HBM: it pulls a solve from the group's job
-// list (atomic ticket), its leader CTA builds the start state, then every
-// iteration the cluster's CTAs evaluate the tiles of the pair space round-robin
+// list (atomic ticket), its leader CTA builds the start state, then the cluster
+// runs the candidate pass (cand.cuh); for pinned sweeps and iterations it leaves
+// the cluster's CTAs evaluate the tiles of the pair space round-robin
 // (tile_eval, the plain kernel's code), meet at a cluster barrier, the leader
 // merges their records through distributed shared memory and decides/applies
 // the move (decide_apply, also the plain kernel's code) and the cluster meets
@@ -399,7 +400,7 @@ ts_status plan_group_st(Group& G, std::vector<BatchJobDev>& table, int64_t budge
   }
 }
 
-// CTAs per solve when the job asks for "auto": a solve whose share of the
+// CTAs per solve of a pinned sweep when the job asks for "auto": a solve whose share of the
 // batch's work would outlast the rest on one CTA is spread over a cluster, so
 // the batch does not end on one long solve.
 int32_t auto_cluster(double work, double total, int sms) {

@@ -9,8 +9,8 @@
 //          width, cluster size) group, one thread-block cluster per solve,
 //          running its iterations with the batched form's device code
 //          (packed.cuh) on state that stays resident between rounds;
-//        - large solves ("plain"): the one-launch-per-iteration kernel of
-//          ts_solver_* on the solve's own stream, using the whole GPU;
+//        - large solves ("plain"): ts_solver_*'s launches on the solve's own
+//          stream (one cluster each, or whole-GPU sweeps);
 //      all groups and plain solves run concurrently on separate streams;
 //   3. collects completed solves (result, best solution), frees their memory.
 // A request that arrives during a round joins at the next one, so short

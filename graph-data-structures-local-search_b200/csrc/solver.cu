@@ -5,9 +5,9 @@
 // host-side init (initialSolution / calculateVertexGain / computeGainsFromScratch,
 // GPU-MDP-CSR.cu:479-519, GPU-MAXBS-CSR.cu:197-219,307-324) runs here as device
 // kernels, and the per-iteration host loop (4-5 launches + a blocking 8-byte D2H
-// per iteration) becomes back-to-back launches of one iteration kernel whose
-// state lives in HBM (sweep.cuh).  The host only touches the device between
-// batches of iterations.
+// per iteration) becomes one cluster launch for many iterations (cand.cuh), or
+// back-to-back launches of one iteration kernel whose state lives in HBM
+// (sweep.cuh).  The host only touches the device between batches of iterations.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>

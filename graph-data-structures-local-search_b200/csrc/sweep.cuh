@@ -1,4 +1,6 @@
-// sweep.cuh -- one tabu iteration as ONE kernel launch.
+// sweep.cuh -- one tabu iteration as ONE kernel launch that visits all pairs:
+// what pinned sweeps run, and the default candidate pass (cand.cuh) for the
+// iterations it does not settle.
 //
 // Replaces, per iteration, the reference's calculateSwapGain / calculateMoveGain
 // (src/mdp/GPU-MDP-CSR.cu:567-584, src/maxbisection/GPU-MAXBS-CSR.cu:337-353 and
