@@ -95,3 +95,28 @@ def test_enqueue_keeps_its_count(gpu, problem):
     assert s.sync() == 40
     s.close()
     g.close()
+
+
+@pytest.mark.parametrize("sweep", [T.PASS_AUTO, T.PASS_TILE])
+@pytest.mark.parametrize("problem", [T.PROBLEM_MDP, T.PROBLEM_MAXBS])
+def test_wswap_started_again(gpu, problem, sweep):
+    """A solver started again (its matrix cleared along the old state's edges)
+    searches as a new one does, with duplicated edges and self-loops too."""
+    n = 400
+    u, v, w = rand_graph(n, 0.05, 21, dup=True, selfloops=problem == T.PROBLEM_MAXBS)
+    g = T.Graph(n, u, v, w, "wswap", drop_self_loops=problem == T.PROBLEM_MDP)
+    kw = dict(m=40 if problem == T.PROBLEM_MDP else 0, max_iter=120, tenure_policy=FIXED, tenure=7, piter=11, gamma=9,
+              sweep=sweep)
+    again = T.Solver(g, problem, **kw)
+    for seed in (1, 2, 3):
+        start = T.random_start(problem, n, kw["m"], seed)
+        new = T.Solver(g, problem, **kw)
+        for s in (again, new):
+            s.init(start)
+            s.step(120)
+        for a, b in zip(again.state(), new.state()):
+            np.testing.assert_array_equal(a, b)
+        assert again.result().best == new.result().best
+        new.close()
+    again.close()
+    g.close()
