@@ -73,7 +73,8 @@ typedef enum ts_tenure { TS_TENURE_REF = 0, TS_TENURE_FIXED = 1 } ts_tenure;
  *   structure (fewer, cheaper tiles: small instances).
  * TS_PASS_AUTO: the candidate pass, which finds the same best pair from the
  *   rows and columns whose bounds can reach it and runs its iterations in one
- *   launch (about 290,000 vertices at most with 32-bit keys).  Iterations it
+ *   launch (up to about 210,000 vertices in Max Bisection and 250,000 in MDP
+ *   with 32-bit keys).  Iterations it
  *   does not settle (ties everywhere, no allowed pair), and larger graphs:
  *   TILE from 2^22 swap pairs per iteration up (CSR with MDP or a negative
  *   weight: ROWS), else ROWS. */
