@@ -13,8 +13,10 @@
 // position-ordered contributions and tabu flags, the positions by vertex, the
 // per-CTA records, the bounds and two last-CTA tickets.  Every GPU that loads
 // the library keeps it until the process exits.  All calls share it and it
-// keeps the last call's contents: the tickets are cleared by every call, and
-// calls that overlap on the GPU (from other streams or host threads) race on it.
+// keeps the last call's contents.  Calls that overlap on the GPU (from other
+// streams or host threads) race on it and decide wrongly; they read and write
+// nothing out of bounds, and leave nothing behind: each launch of a call clears
+// the other launch's ticket, so that later calls count from 0 again.
 //
 // Cost: the pairs are bounded as in the solver's candidate pass (cand.cuh).
 // One launch orders the state, takes the maxima of both sides and of the
@@ -109,6 +111,7 @@ k_na_stage(int32_t problem, int32_t n, int32_t m, long long iter, long long D, c
   __shared__ CtaRec s_top[5];
   __shared__ int32_t s_last;
   const int tid = threadIdx.x;
+  if (blockIdx.x == 0 && tid == 0) *sc.counter = 0u;
   const long long stride = (long long)gridDim.x * blockDim.x;
   long long k4[4], i4[4];
 #pragma unroll
@@ -129,10 +132,7 @@ k_na_stage(int32_t problem, int32_t n, int32_t m, long long iter, long long D, c
     for (int q = 0; q < 4; q++)
       if ((q < 2) == row && ((q & 1) || !t)) better_rec(k4[q], i4[q], y, p);
   }
-  if constexpr (!BOUNDS) {
-    if (blockIdx.x == 0 && tid == 0) *sc.counter = 0u;
-    return;
-  }
+  if constexpr (!BOUNDS) return;
   // the weights' range, as records of (max, .) and (-min, .)
   long long hi = 0, lo = 0;
   const long long E = rowptr[n];
@@ -191,7 +191,10 @@ k_na_stage(int32_t problem, int32_t n, int32_t m, long long iter, long long D, c
   // c*w of the pairs of the maxima 0, 2 and 1, 3: a warp each
   if (tid < 64 && (tid >= 32 || nt_ok)) {
     const int q = tid >> 5;
-    const long long x = na_warp_lookup(rowptr, col, w, sol[s_top[q].idx], sol[s_top[q + 2].idx]);
+    // (records of an overlapping call may hold positions of its larger state)
+    const long long i = s_top[q].idx, j = s_top[q + 2].idx;
+    const bool in = i >= 0 && i < n && j >= 0 && j < n;
+    const long long x = in ? na_warp_lookup(rowptr, col, w, sol[i], sol[j]) : 0;
     if ((tid & 31) == 0) red[q].key = problem == P_MDP ? -x : 2 * x;
   }
   __syncthreads();
@@ -221,7 +224,6 @@ k_na_stage(int32_t problem, int32_t n, int32_t m, long long iter, long long D, c
   g.need_n = (nt_ok && c1 < 0 && Am + Bm >= g.LB) || (c2 < 0 && AA + BA >= g.LT);
   *sc.goal = g;
   *sc.staged = 0u;
-  *sc.counter = 0u;
 }
 
 // First entry of u's sorted row with neighbour v (lower_bound), else 0.
@@ -248,6 +250,7 @@ k_na_sweep(int32_t problem, int32_t n, int32_t m, long long cur, long long best,
   const int32_t delta = n - m;
   const long long P = (long long)m * delta;
   const long long D = best - cur;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *sc.staged = 0u;  // after an overlap it may have passed its mark
   long long bk = LLONG_MIN, bi = LLONG_MAX;
   if (BOUNDS && !sc.goal->all_pairs) {
     const NaGoal g = *sc.goal;
