@@ -288,7 +288,7 @@ __global__ void k_init_maxbs(const DevGraph g, const DevSolver<KeyT> s, unsigned
     for (long long k = g.rowptr[z] + lane; k < g.rowptr[z + 1]; k += 32) {
       const int2 e = g.adj[k];
       const bool sy = s.pos[e.x] < s.m;
-      gain += sy == side ? e.y : -e.y;
+      gain += sy == side ? e.y : -(long long)e.y;  // (-2^31 has no 32-bit negative)
       if (sy != side && e.x > z) c += e.y;
     }
 #pragma unroll
