@@ -49,6 +49,7 @@ constexpr int kCandStage = 1024;     // candidate columns staged per round of N
 constexpr int kCandHeavy = 512;      // E: rows of more entries are walked by the whole CTA
 constexpr int kCandHeavyList = 64;
 constexpr int kCandHits = 2048;      // E: entries kept for evaluation per round (more: a sweep)
+constexpr int kCandRowBits = 22;     // E: a kept entry's place in its row, beside 9 bits for the row
 constexpr int kCandGroupPairs = 12;  // N: up to this many pairs a warp, eight lanes look each one up
 
 enum { kCandEnd = 0, kCandBail = 1 };
@@ -773,6 +774,10 @@ __device__ int cand_run(const DevGraph& g, const DevSolver<KeyT>& s, long long s
             const KeyT fn = dn + sh.goal.s_nt, fa = da + sh.goal.s_all;
             const KeyT f = dn <= q_nt && (da > q_all || fn < fa) ? fn : fa;
             if ((PROB == P_MDP ? -(KeyT)wr.x : (KeyT)2 * (KeyT)wr.y) < f) l = 0;  // no entry weighs enough
+            if (l > 1 << kCandRowBits) {  // (parallel edges) counts as too many kept entries: a sweep
+              atomicAdd(&sh.nhits, kCandHits + 1);
+              l = 0;
+            }
             if (l > kCandHeavy) {
               const int32_t at = atomicAdd(&sh.nheavy, 1);
               if (at < kCandHeavyList) {
@@ -864,7 +869,7 @@ __device__ int cand_run(const DevGraph& g, const DevSolver<KeyT>& s, long long s
             for (int x = 0; x < 8; x++) {
               if (e[x].x < 0) continue;
               const KeyT c = PROB == P_MDP ? -(KeyT)e[x].y : (KeyT)2 * (KeyT)e[x].y;
-              if (c >= least[r[x]] && (map[e[x].x >> 5] >> (e[x].x & 31) & 1u) && k[x] < (1 << 22)) keep |= 1u << x;
+              if (c >= least[r[x]] && (map[e[x].x >> 5] >> (e[x].x & 31) & 1u)) keep |= 1u << x;
             }
             if (!__any_sync(0xffffffffu, keep)) continue;
             int32_t pre = __popc(keep);

@@ -1,4 +1,6 @@
-"""Inputs at the ends of their ranges, against the CPU oracle."""
+"""Inputs at the ends of their ranges, against the CPU oracle: the lowest
+32-bit weight, and a row of more entries than a packed queue word can number.
+"""
 import numpy as np
 import pytest
 
@@ -37,3 +39,31 @@ def test_lowest_weight_batched(gpu, problem):
         assert (r.iterations, r.cur, r.best, r.best_true, r.device_error) == (o.iterations, o.cur, o.best, o.best_true, 0)
     for g in graphs:
         g.close()
+
+
+def long_row_graph(problem):
+    """2^22 + 9 parallel edges 0-1 of weight 0, so that vertex 0's other
+    neighbours lie beyond the 2^22-th entry of its row, and weights for which
+    the best swap is (0, 40), an adjacent pair that only row 0 leads to: column
+    40 is further from its side's best than half of what the pair's weight
+    makes up."""
+    n, few = 64, 2 ** 22 + 9
+    if problem == T.PROBLEM_MAXBS:  # part 0: vertices 0-31
+        rest = [(0, k, 100) for k in range(2, 12)] + [(0, 40, 100), (50, 51, 50)]
+    else:  # inside: 0-31; contributions are weighted degrees into the set
+        rest = [(k, j, 100) for k in range(1, 32) for j in range(k + 1, 32)] + \
+               [(50, k, 90) for k in range(1, 4)] + [(40, 1, 300), (0, 40, -100)]
+    ru, rv, rw = (np.array(x, np.int32) for x in zip(*rest))
+    u = np.concatenate([np.zeros(few, np.int32), ru])
+    v = np.concatenate([np.ones(few, np.int32), rv])
+    w = np.concatenate([np.zeros(few, np.int32), rw])
+    initial = np.arange(32, dtype=np.int32) if problem == T.PROBLEM_MDP else (np.arange(n) >= 32).astype(np.int32)
+    return n, u, v, w, initial
+
+
+@pytest.mark.parametrize("kind", ["csr", "csr-bb", "hash", "wswap"])
+@pytest.mark.parametrize("problem", [T.PROBLEM_MDP, T.PROBLEM_MAXBS])
+def test_row_of_more_than_2_to_22_entries(gpu, problem, kind):
+    n, u, v, w, initial = long_row_graph(problem)
+    compare_run(problem, kind, n, u, v, w, m=32 if problem == T.PROBLEM_MDP else 0, iters=6, tenure_policy=FIXED, tenure=3,
+                initial=initial)
