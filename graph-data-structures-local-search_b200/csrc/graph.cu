@@ -35,95 +35,152 @@ ts_status cuda_fail(cudaError_t e, const char* what) {
   return e == cudaErrorMemoryAllocation ? TS_ERR_OUT_OF_MEMORY : TS_ERR_CUDA;
 }
 
-namespace {
-constexpr int kMaxDevices = 64;
-struct Pool {
-  cudaMemPool_t pool = nullptr;
-  cudaStream_t stream = nullptr;  // allocations and frees for any stream
-  bool tried = false;
-  int users = 0;
-};
-std::mutex g_pool_mu;
-Pool g_pool[kMaxDevices];
-
-// The current device's pool; without one (old driver) plain allocations are used.
-Pool* device_pool() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
-  std::lock_guard<std::mutex> lock(g_pool_mu);
-  Pool& t = g_pool[dev];
-  if (!t.tried) {
-    t.tried = true;
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.handleTypes = cudaMemHandleTypeNone;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    uint64_t keep = kPoolKeep;
-    if (cudaStreamCreateWithFlags(&t.stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMemPoolCreate(&t.pool, &props) != cudaSuccess) {
-      t.pool = nullptr;
+uint64_t context_id() {
+  // Reached through the runtime, so that the library needs no link-time
+  // dependency on the driver library.
+  using GetCurrent = int (*)(void**);
+  using GetId = int (*)(void*, unsigned long long*);
+  struct Driver {
+    GetCurrent current = nullptr;
+    GetId id = nullptr;
+  };
+  static const Driver d = [] {
+    Driver f;
+    auto find = [](const char* name) {
+      void* fn = nullptr;
+      cudaDriverEntryPointQueryResult q;
+      if (cudaGetDriverEntryPoint(name, &fn, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) {
+        cudaGetLastError();
+        fn = nullptr;
+      }
+      return fn;
+    };
+    f.current = reinterpret_cast<GetCurrent>(find("cuCtxGetCurrent"));
+    f.id = reinterpret_cast<GetId>(find("cuCtxGetId"));
+    return f;
+  }();
+  void* ctx = nullptr;
+  unsigned long long id = 0;
+  if (!d.current || !d.id || d.current(&ctx) != 0) return 0;
+  if (!ctx || d.id(ctx, &id) != 0) {
+    // none bound to this thread yet, or one that a reset has ended: the
+    // device's primary context, the one the runtime would use
+    int dev = 0;
+    id = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess || d.current(&ctx) != 0 || !ctx ||
+        d.id(ctx, &id) != 0) {
       cudaGetLastError();
-    } else {
-      cudaMemPoolSetAttribute(t.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      return 0;
     }
   }
-  return t.pool ? &t : nullptr;
+  return id;
+}
+
+// One pool per context: a context that ends (a device reset) takes its pool,
+// stream and memory along, and the next one gets a pool of its own.  Entries
+// of ended contexts stay, so that an entry's address says which context a
+// block belongs to.
+struct Pool {
+  uint64_t ctx = 0;
+  cudaMemPool_t pool = nullptr;
+  cudaStream_t stream = nullptr;  // allocations and frees for any stream
+  int users = 0;
+};
+
+namespace {
+constexpr int kMaxPools = 64;
+std::mutex g_pool_mu;
+Pool g_pool[kMaxPools];
+int g_pools = 0;
+
+// The current context's pool; null (no context ids, no pool to be had, or 64
+// contexts before this one): plain allocations.
+Pool* context_pool() {
+  const uint64_t ctx = context_id();
+  if (!ctx) return nullptr;
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  for (int k = 0; k < g_pools; k++)
+    if (g_pool[k].ctx == ctx) return g_pool[k].pool ? &g_pool[k] : nullptr;
+  if (g_pools == kMaxPools) return nullptr;
+  Pool& t = g_pool[g_pools++];
+  t.ctx = ctx;
+  int dev = 0;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.handleTypes = cudaMemHandleTypeNone;
+  props.location.type = cudaMemLocationTypeDevice;
+  uint64_t keep = kPoolKeep;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaStreamCreateWithFlags(&t.stream, cudaStreamNonBlocking) != cudaSuccess ||
+      (props.location.id = dev, cudaMemPoolCreate(&t.pool, &props)) != cudaSuccess) {
+    t.pool = nullptr;
+    cudaGetLastError();
+    return nullptr;
+  }
+  cudaMemPoolSetAttribute(t.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  return &t;
+}
+
+// Tried again once what the pool holds unused has been given back.
+template <class Get>
+cudaError_t with_trim(Get&& get) {
+  cudaError_t e = get();
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  pool_trim();
+  return get();
 }
 }  // namespace
 
-cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st) {
-  *p = nullptr;
-  Pool* t = device_pool();
-  for (int attempt = 0;; attempt++) {
-    const cudaError_t e = t ? cudaMallocFromPoolAsync(p, bytes, t->pool, st) : cudaMallocAsync(p, bytes, st);
-    if (e != cudaErrorMemoryAllocation || attempt) return e;
-    cudaGetLastError();
-    pool_trim();
+cudaError_t pool_get(PoolBlock& b, size_t bytes, bool ordered, cudaStream_t st) {
+  b = PoolBlock{};
+  b.ctx = context_id();
+  b.ordered = ordered;
+  b.stream = st;
+  Pool* t = context_pool();
+  cudaError_t e;
+  if (!t || (!ordered && bytes > kPoolBlock)) {
+    e = with_trim([&] { return cudaMalloc(&b.p, bytes); });
+  } else {
+    b.pool = t;
+    if (!ordered) b.stream = t->stream;
+    e = with_trim([&] { return cudaMallocFromPoolAsync(&b.p, bytes, t->pool, b.stream); });
+    if (e == cudaSuccess && !ordered) e = cudaStreamSynchronize(b.stream);
   }
+  if (e != cudaSuccess) b.p = nullptr;
+  return e;
 }
-void pool_free(void* p, cudaStream_t st) {
-  if (p) cudaFreeAsync(p, st);
-}
-cudaError_t pool_get(void** p, size_t bytes) {
-  Pool* t = device_pool();
-  if (bytes > kPoolBlock) {
-    for (int attempt = 0;; attempt++) {
-      const cudaError_t e = cudaMalloc(p, bytes);
-      if (e != cudaErrorMemoryAllocation || attempt) return e;
-      cudaGetLastError();
-      pool_trim();
+void pool_put(PoolBlock& b) {
+  if (b.p && context_id() == b.ctx) {  // else its context has ended, and the memory with it
+    if (!b.pool) {
+      if (b.ordered) cudaStreamSynchronize(b.stream);
+      cudaFree(b.p);
+    } else {
+      if (!b.ordered) cudaDeviceSynchronize();
+      cudaFreeAsync(b.p, b.stream);
     }
   }
-  const cudaStream_t st = t ? t->stream : nullptr;
-  const cudaError_t e = pool_alloc(p, bytes, st);
-  return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
-}
-void pool_put(void* p, size_t bytes) {
-  if (!p) return;
-  if (bytes > kPoolBlock) {
-    cudaFree(p);
-    return;
-  }
-  Pool* t = device_pool();
-  cudaDeviceSynchronize();
-  cudaFreeAsync(p, t ? t->stream : nullptr);
+  b = PoolBlock{};
 }
 void pool_trim() {
-  Pool* t = device_pool();
+  Pool* t = context_pool();
   if (!t) return;
   cudaDeviceSynchronize();  // frees still queued on a stream
   cudaMemPoolTrimTo(t->pool, 0);
 }
-void pool_users(int device, int change) {
-  if (device < 0 || device >= kMaxDevices) return;
-  cudaMemPool_t idle = nullptr;
+Pool* pool_enter() {
+  Pool* t = context_pool();
+  if (!t) return nullptr;
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  t->users++;
+  return t;
+}
+void pool_leave(Pool* t) {
+  if (!t) return;
   {
     std::lock_guard<std::mutex> lock(g_pool_mu);
-    g_pool[device].users += change;
-    if (change < 0 && g_pool[device].users == 0) idle = g_pool[device].pool;
+    if (--t->users > 0) return;
   }
-  if (idle) cudaMemPoolTrimTo(idle, kPoolIdle);
+  if (context_id() == t->ctx) cudaMemPoolTrimTo(t->pool, kPoolIdle);
 }
 
 cudaError_t allow_dyn_smem(const void* fn, size_t smem) {
@@ -562,7 +619,7 @@ static ts_status make_graph(int32_t n, int64_t E, const int32_t* u, const int32_
   cudaGetDevice(&G->device);
   ts_status s = build_graph(G, E, u, v, w, on_host);
   if (s != TS_OK) { delete G; return s; }
-  pool_users(G->device, 1);
+  G->pool = pool_enter();
   *out = G;
   return TS_OK;
 }
@@ -632,9 +689,10 @@ ts_status ts_graph_destroy(ts_graph* g) {
   if (!g) return TS_OK;
   cudaSetDevice(g->device);
   cudaStreamSynchronize(g->stream);
-  const int device = g->device;
+  Pool* pool = g->pool;
   delete g;
-  pool_users(device, -1);
+  pool_leave(pool);
+  cudaGetLastError();  // a context that ended before its graph: no error for the next call to find
   return TS_OK;
 }
 

@@ -1186,6 +1186,7 @@ ts_status ts_solver_destroy(ts_solver* s) {
   cudaStreamSynchronize(s->g->stream);
   if (s->h_st) cudaFreeHost(s->h_st);
   delete s;
+  cudaGetLastError();  // (as in ts_graph_destroy)
   return TS_OK;
 }
 

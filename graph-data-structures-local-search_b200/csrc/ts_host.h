@@ -38,27 +38,39 @@ ts_status cuda_fail(cudaError_t e, const char* what);
     if (e_ != cudaSuccess) return ::tsb::cuda_fail(e_, #call); \
   } while (0)
 
+// Identity of the context current on the calling thread (the device's primary
+// context if none is); 0 when the driver does not tell.  Unlike the context's
+// address it does not come back after a device reset.
+uint64_t context_id();
+
 // Device memory of graphs, solvers and calls comes from a memory pool of the
-// library's own per device: outside a pool an allocation or free of megabytes
+// library's own per context: outside a pool an allocation or free of megabytes
 // costs 50 us to milliseconds and stalls every stream (ER n = 2,000: graph
 // 650 -> 150 us, its and its solver's end 450 -> 30 us).  The pool keeps at
 // most kPoolKeep unused bytes, kPoolIdle once the last graph is gone, and
-// nothing when an allocation of the library finds no memory.  Blocks above
+// gives them back before an allocation of the library fails.  Blocks above
 // kPoolBlock that outlive a call are plain allocations: the pool grows and
 // shrinks by many small mappings (a matrix of 1.8 GB: 10 ms and more, 0.5 ms
 // plain).
-//   pool_alloc/pool_free   in stream order (temporaries of one call);
-//   pool_get/pool_put      for any stream: ready on return; put waits for the
-//                          device, as a plain free does.
 constexpr size_t kPoolKeep = 512u << 20;
 constexpr size_t kPoolIdle = 256u << 20;
 constexpr size_t kPoolBlock = 64u << 20;
-cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t st);
-void pool_free(void* p, cudaStream_t st);
-cudaError_t pool_get(void** p, size_t bytes);
-void pool_put(void* p, size_t bytes);
-void pool_trim();                         // current device: unused bytes back to the driver
-void pool_users(int device, int change);  // graphs alive on the device
+struct Pool;
+struct PoolBlock {
+  void* p = nullptr;
+  uint64_t ctx = 0;      // the context it lives in
+  Pool* pool = nullptr;  // null: a plain allocation
+  bool ordered = false;  // for work on `stream` alone, freed in its order
+  cudaStream_t stream = nullptr;
+};
+// ordered: for work on `st` alone (temporaries of one call); else for any
+// stream: ready on return, and pool_put waits for the device, as a plain free
+// does.
+cudaError_t pool_get(PoolBlock& b, size_t bytes, bool ordered, cudaStream_t st);
+void pool_put(PoolBlock& b);
+void pool_trim();           // current context: unused bytes back to the driver
+Pool* pool_enter();         // a graph begins: the current context's pool
+void pool_leave(Pool* pool);  // and ends
 
 // Owning device buffer.
 struct DevBuf {
@@ -101,43 +113,29 @@ struct DevPart {
 // Parts of one pool allocation: sizes are registered first, then placed
 // together (every part starts on 256 bytes).
 struct DevParts {
-  void* mem = nullptr;
-  size_t bytes = 0;
-  bool ordered = false;  // freed in the order of `stream`
-  cudaStream_t stream = nullptr;
+  PoolBlock mem;
   std::vector<std::pair<DevPart*, size_t>> parts;
   DevParts() = default;
   DevParts(const DevParts&) = delete;
   DevParts& operator=(const DevParts&) = delete;
-  ~DevParts() {
-    if (!mem) return;
-    if (ordered) pool_free(mem, stream);
-    else pool_put(mem, bytes);
-  }
+  ~DevParts() { pool_put(mem); }
   void add(DevPart& part, size_t n) {
     part.bytes = n;
     parts.emplace_back(&part, n);
   }
   // For any stream, until the object goes.
-  ts_status alloc(const char* what) { return place(what); }
+  ts_status alloc(const char* what) { return place(what, false, nullptr); }
   // For work on `st` alone.
-  ts_status alloc_temp(const char* what, cudaStream_t st) {
-    ordered = true;
-    stream = st;
-    return place(what);
-  }
+  ts_status alloc_temp(const char* what, cudaStream_t st) { return place(what, true, st); }
 
  private:
-  ts_status place(const char* what) {
+  ts_status place(const char* what, bool ordered, cudaStream_t st) {
     auto pad = [](size_t b) { return b ? (b + 255) & ~(size_t)255 : (size_t)256; };
-    bytes = 0;
+    size_t bytes = 0;
     for (auto& x : parts) bytes += pad(x.second);
-    const cudaError_t e = ordered ? pool_alloc(&mem, bytes, stream) : pool_get(&mem, bytes);
-    if (e != cudaSuccess) {
-      mem = nullptr;
-      return cuda_fail(e, what);
-    }
-    unsigned char* p = static_cast<unsigned char*>(mem);
+    const cudaError_t e = pool_get(mem, bytes, ordered, st);
+    if (e != cudaSuccess) return cuda_fail(e, what);
+    unsigned char* p = static_cast<unsigned char*>(mem.p);
     for (auto& x : parts) {
       x.first->p = p;
       p += pad(x.second);
@@ -162,6 +160,7 @@ struct ts_graph {
   int64_t max_abs_w = 0;  // largest |w| of an entry
   int64_t wpr = 0;
   int64_t hash_slots = 0;
+  tsb::Pool* pool = nullptr;  // entered by the graph
   tsb::DevParts mem, tables;  // what is known before the sort; the hash tables
   tsb::DevPart rowptr, adj, bits, hoff, hkey, hval, rev, wrange;
   // Host copy of the CSR row pointers/degrees (for footprint planning and the
