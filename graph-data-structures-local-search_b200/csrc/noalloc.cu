@@ -327,31 +327,15 @@ k_na_sweep(int32_t problem, int32_t n, int32_t m, long long cur, long long best,
 constexpr int kMaxDevices = 64;
 std::mutex g_na_mu;
 // The scratch array has one address per CUDA context: cached per device
-// together with the context it was looked up in, and looked up again when the
-// caller's current context on that device is another one (a context the caller
-// created itself, or a new primary context after a device reset).
+// together with the id of the context it was looked up in, and looked up again
+// when the caller's current context on that device is another one (a context
+// the caller created itself, or a new primary context after a device reset,
+// which may have the old one's address but not its id).
 struct NaAddr {
-  void* ctx;
+  uint64_t ctx;
   void* addr;
 };
 NaAddr g_na_addr[kMaxDevices];
-
-// cuCtxGetCurrent, reached through the runtime so the library needs no
-// link-time dependency on the driver library.
-using CtxGetCurrentFn = int (*)(void**);
-CtxGetCurrentFn ctx_get_current() {
-  static CtxGetCurrentFn fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess) {
-      cudaGetLastError();
-      f = nullptr;
-    }
-    return reinterpret_cast<CtxGetCurrentFn>(f);
-  }();
-  return fn;
-}
 
 }  // namespace
 }  // namespace tsb
@@ -386,20 +370,10 @@ extern "C" ts_status ts_best_swap_noalloc(int32_t problem, int32_t n, int32_t m,
     // the current context (its name in host code is only a host-side
     // stand-in).  The first call in a context looks it up; later calls in the
     // same context reuse it.
-    CtxGetCurrentFn get_ctx = ctx_get_current();
-    if (!get_ctx) {
-      set_error("ts_best_swap_noalloc: cuCtxGetCurrent is not available from the driver");
-      return TS_ERR_UNSUPPORTED;
-    }
-    void* ctx = nullptr;
-    if (get_ctx(&ctx) != 0 || !ctx) {
-      // No context bound to this thread yet: bind the device's primary context
-      // (cudaSetDevice initialises it) -- the one the runtime would use.
-      TS_CUDA(cudaSetDevice(dev));
-      if (get_ctx(&ctx) != 0 || !ctx) {
-        set_error("ts_best_swap_noalloc: no current CUDA context on the calling thread");
-        return TS_ERR_CUDA;
-      }
+    const uint64_t ctx = context_id();
+    if (!ctx) {
+      set_error("ts_best_swap_noalloc: no current CUDA context on the calling thread");
+      return TS_ERR_CUDA;
     }
     std::lock_guard<std::mutex> lock(g_na_mu);
     if (g_na_addr[dev].ctx != ctx || !g_na_addr[dev].addr) {
