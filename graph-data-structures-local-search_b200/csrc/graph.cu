@@ -120,14 +120,17 @@ Pool* context_pool() {
   return &t;
 }
 
-// Tried again once what the pool holds unused has been given back.
+// Tried again once what the pool holds unused has been given back; a pool that
+// still does not get what it needs gives back what it got.
 template <class Get>
 cudaError_t with_trim(Get&& get) {
-  cudaError_t e = get();
-  if (e != cudaErrorMemoryAllocation) return e;
-  cudaGetLastError();
-  pool_trim();
-  return get();
+  for (int attempt = 0;; attempt++) {
+    const cudaError_t e = get();
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    pool_trim();
+    if (attempt) return e;
+  }
 }
 }  // namespace
 
@@ -301,13 +304,28 @@ k_max_wdeg(int32_t n, const int64_t* __restrict__ rowptr, const int2* __restrict
   }
 }
 
-__global__ void k_fill_bits(int32_t n, int cb, int64_t N2, const unsigned long long* __restrict__ keys, int64_t wpr,
+// Row of entry k: from its sorted key, or, where the keys had to make room for
+// the graph (keys null), the last row that starts at or before k.
+__device__ __forceinline__ int64_t row_of(int32_t n, int cb, const unsigned long long* __restrict__ keys,
+                                          const int64_t* __restrict__ rowptr, int64_t k) {
+  if (keys) return (int64_t)(keys[k] >> cb);
+  int32_t lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int32_t mid = (lo + hi + 1) >> 1;
+    if (rowptr[mid] <= k) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+__global__ void k_fill_bits(int32_t n, int cb, int64_t N2, const unsigned long long* __restrict__ keys,
+                            const int64_t* __restrict__ rowptr, const int2* __restrict__ adj, int64_t wpr,
                             unsigned long long* __restrict__ bits) {
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < N2;
        k += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = (int64_t)(keys[k] >> cb);
-    const int32_t c = (int32_t)(keys[k] & ((1ull << cb) - 1));
-    if (r < n) atomicOr(&bits[r * wpr + (c >> 6)], 1ull << (c & 63));
+    const int64_t r = row_of(n, cb, keys, rowptr, k);
+    if (r >= n) continue;
+    const int32_t c = keys ? (int32_t)(keys[k] & ((1ull << cb) - 1)) : adj[k].x;
+    atomicOr(&bits[r * wpr + (c >> 6)], 1ull << (c & 63));
   }
 }
 
@@ -318,13 +336,13 @@ __global__ void k_hash_caps(int32_t n, const int64_t* __restrict__ rowptr, int64
 }
 
 // Inserts the first entry of every (row, neighbour) pair with linear probing.
-__global__ void k_hash_insert(int cb, int64_t N, const unsigned long long* __restrict__ sorted,
+__global__ void k_hash_insert(int32_t n, int cb, int64_t N, const unsigned long long* __restrict__ sorted,
                               const int64_t* __restrict__ rowptr, const int2* __restrict__ adj, const int64_t* __restrict__ hoff,
                               int32_t* __restrict__ keys, int32_t* __restrict__ vals,
                               int32_t* __restrict__ err) {
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < N;
        k += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = (int64_t)(sorted[k] >> cb);
+    const int64_t r = row_of(n, cb, sorted, rowptr, k);
     int2 e = adj[k];
     if (k > rowptr[r] && adj[k - 1].x == e.x) continue;  // duplicate pair: first wins
     const int64_t base = hoff[r];
@@ -354,7 +372,7 @@ __global__ void k_reverse_index(int32_t n, int cb, int64_t N2, const unsigned lo
                                 int64_t* __restrict__ rev) {
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < N2;
        k += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = (int64_t)(keys[k] >> cb);
+    const int64_t row = row_of(n, cb, keys, rowptr, k);
     if (row >= n) continue;
     const int32_t y = (int32_t)row;
     const int32_t z = adj[k].x;
@@ -447,6 +465,10 @@ __global__ void k_lookup(DevGraph g, int64_t count, const int32_t* __restrict__ 
 // each.  One host round trip, two for Hash.  Conflict graph, n = 100,000, 3.4M
 // edges, from host arrays: Hash 11.2 -> 5.3 ms (2.3 of them the copies), CSR
 // 8.7 -> 5.2; a million lookups 3.3 -> 1.1 ms.
+// Where the device has no room for the temporaries (48 bytes an edge) beside
+// all of the graph, only what the sort fills is allocated with them, and the
+// bitmap, the reverse index or the hash tables once they are gone; these are
+// then filled from the rows, with a search for each entry's row.
 static ts_status build_graph(ts_graph* G, int64_t E, const int32_t* u, const int32_t* v, const int32_t* w,
                              bool on_host) {
   cudaStream_t st = G->stream;
@@ -459,16 +481,16 @@ static ts_status build_graph(ts_graph* G, int64_t E, const int32_t* u, const int
   while ((1LL << row_bits) <= (int64_t)n) row_bits++;
   while ((1LL << cb) < (int64_t)n) cb++;
   ts_status s;
-  DevParts temp;
-  DevPart keys, keys_alt, vals, vals_alt, sum, tmp, caps;
+  auto temp = std::make_unique<DevParts>();
+  DevPart keys, keys_alt, vals, vals_alt, sum, tmp, caps, full;
   const size_t eb = sizeof(int32_t) * (size_t)E;
-  temp.add(keys, sizeof(unsigned long long) * N2);
-  temp.add(keys_alt, sizeof(unsigned long long) * N2);
-  temp.add(vals, sizeof(int32_t) * N2);
-  temp.add(vals_alt, sizeof(int32_t) * N2);
+  temp->add(keys, sizeof(unsigned long long) * N2);
+  temp->add(keys_alt, sizeof(unsigned long long) * N2);
+  temp->add(vals, sizeof(int32_t) * N2);
+  temp->add(vals_alt, sizeof(int32_t) * N2);
   // sum: wdeg results (3 words), then the error word
-  temp.add(sum, 4 * sizeof(unsigned long long));
-  if (hash) temp.add(caps, sizeof(int64_t) * (n + 1));
+  temp->add(sum, 4 * sizeof(unsigned long long));
+  if (hash) temp->add(caps, sizeof(int64_t) * (n + 1));
   size_t sort_bytes = 0, scan_bytes = 0;
   {
     cub::DoubleBuffer<unsigned long long> dk;
@@ -477,22 +499,35 @@ static ts_status build_graph(ts_graph* G, int64_t E, const int32_t* u, const int
     int64_t* none = nullptr;
     if (hash) TS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, none, none, n + 1, st));
   }
-  temp.add(tmp, sort_bytes > scan_bytes ? sort_bytes : scan_bytes);
-  if ((s = temp.alloc_temp("alloc build temporaries", st)) != TS_OK) return s;
+  temp->add(tmp, sort_bytes > scan_bytes ? sort_bytes : scan_bytes);
+  if ((s = temp->alloc_temp("alloc build temporaries", st)) != TS_OK) return s;
 
-  G->mem.add(G->rowptr, sizeof(int64_t) * (n + 1));
-  // Two spare entries: the sweep bulk-copies rows from an even entry to an
-  // even end (16-byte aligned), which can reach one entry past the last row.
-  G->mem.add(G->adj, sizeof(int2) * (N2 + 2));
-  G->mem.add(G->wrange, sizeof(int2) * (size_t)n);
-  if (bitset) {
-    const int64_t words = ((int64_t)n + 63) / 64;
-    G->wpr = (words + 1) & ~1LL;  // even: every row starts on a 16 B boundary
-    G->mem.add(G->bits, sizeof(uint64_t) * (size_t)n * (size_t)G->wpr);
+  auto rows = [&] {
+    G->mem.add(G->rowptr, sizeof(int64_t) * (n + 1));
+    // Two spare entries: the sweep bulk-copies rows from an even entry to an
+    // even end (16-byte aligned), which can reach one entry past the last row.
+    G->mem.add(G->adj, sizeof(int2) * (N2 + 2));
+    G->mem.add(G->wrange, sizeof(int2) * (size_t)n);
+    if (hash) G->mem.add(G->hoff, sizeof(int64_t) * (n + 1));
+  };
+  auto filled = [&](DevParts& mem) {  // from the rows; with the hash tables' turn below
+    if (bitset) {
+      const int64_t words = ((int64_t)n + 63) / 64;
+      G->wpr = (words + 1) & ~1LL;  // even: every row starts on a 16 B boundary
+      mem.add(G->bits, sizeof(uint64_t) * (size_t)n * (size_t)G->wpr);
+    }
+    if (G->kind == TS_STRUCT_CSR) mem.add(G->rev, sizeof(int64_t) * (size_t)(N2 > 0 ? N2 : 1));
+  };
+  bool later = false;
+  rows();
+  filled(G->mem);
+  s = G->mem.alloc("alloc graph");
+  if (s == TS_ERR_OUT_OF_MEMORY && (bitset || G->kind == TS_STRUCT_CSR)) {
+    later = true;
+    rows();
+    s = G->mem.alloc("alloc graph");
   }
-  if (hash) G->mem.add(G->hoff, sizeof(int64_t) * (n + 1));
-  if (G->kind == TS_STRUCT_CSR) G->mem.add(G->rev, sizeof(int64_t) * (size_t)(N2 > 0 ? N2 : 1));
-  if ((s = G->mem.alloc("alloc graph")) != TS_OK) return s;
+  if (s != TS_OK) return s;
 
   auto* d_sum = sum.as<unsigned long long>();
   auto* d_err = reinterpret_cast<int32_t*>(d_sum + 3);
@@ -525,18 +560,23 @@ static ts_status build_graph(ts_graph* G, int64_t E, const int32_t* u, const int
   k_max_wdeg<<<blocks_for((int64_t)n * 32), kTPB, 0, st>>>(n, G->rowptr.as<int64_t>(), G->adj.as<int2>(), d_sum,
                                                             G->wrange.as<int2>());
   TS_CUDA(cudaGetLastError());
-  if (bitset) {
-    TS_CUDA(cudaMemsetAsync(G->bits.p, 0, G->bits.bytes, st));
-    if (E > 0) {
-      k_fill_bits<<<blocks_for(N2), kTPB, 0, st>>>(n, cb, N2, dk.Current(), G->wpr, G->bits.as<unsigned long long>());
+  auto fill = [&](int64_t count, const unsigned long long* sorted) -> ts_status {
+    if (bitset) {
+      TS_CUDA(cudaMemsetAsync(G->bits.p, 0, G->bits.bytes, st));
+      if (count > 0) {
+        k_fill_bits<<<blocks_for(count), kTPB, 0, st>>>(n, cb, count, sorted, G->rowptr.as<int64_t>(), G->adj.as<int2>(),
+                                                        G->wpr, G->bits.as<unsigned long long>());
+        TS_CUDA(cudaGetLastError());
+      }
+    }
+    if (G->kind == TS_STRUCT_CSR && count > 0) {
+      k_reverse_index<<<blocks_for(count), kTPB, 0, st>>>(n, cb, count, sorted, G->rowptr.as<int64_t>(),
+                                                          G->adj.as<int2>(), G->rev.as<int64_t>());
       TS_CUDA(cudaGetLastError());
     }
-  }
-  if (G->kind == TS_STRUCT_CSR && E > 0) {
-    k_reverse_index<<<blocks_for(N2), kTPB, 0, st>>>(n, cb, N2, dk.Current(), G->rowptr.as<int64_t>(),
-                                                     G->adj.as<int2>(), G->rev.as<int64_t>());
-    TS_CUDA(cudaGetLastError());
-  }
+    return TS_OK;
+  };
+  if (!later && (s = fill(N2, dk.Current())) != TS_OK) return s;
   int64_t slots = 0;
   if (hash) {
     k_hash_caps<<<blocks_for(n), kTPB, 0, st>>>(n, G->rowptr.as<int64_t>(), caps.as<int64_t>());
@@ -561,24 +601,43 @@ static ts_status build_graph(ts_graph* G, int64_t E, const int32_t* u, const int
   G->max_abs_w = (int64_t)got[2];
   if (hash) {
     G->hash_slots = slots;
-    G->tables.add(G->hkey, sizeof(int32_t) * slots);
-    G->tables.add(G->hval, sizeof(int32_t) * slots);
-    if ((s = G->tables.alloc("alloc hash tables")) != TS_OK) return s;
+    auto tables = [&] {
+      G->tables.add(G->hkey, sizeof(int32_t) * slots);
+      G->tables.add(G->hval, sizeof(int32_t) * slots);
+      G->tables.add(full, sizeof(int32_t));
+      return G->tables.alloc("alloc hash tables");
+    };
+    const unsigned long long* sorted = dk.Current();
+    s = tables();
+    if (s == TS_ERR_OUT_OF_MEMORY) {
+      temp.reset();
+      sorted = nullptr;
+      s = tables();
+    }
+    if (s != TS_OK) return s;
     TS_CUDA(cudaMemsetAsync(G->hkey.p, 0xff, G->hkey.bytes, st));  // kHashEmpty
     TS_CUDA(cudaMemsetAsync(G->hval.p, 0, G->hval.bytes, st));
+    TS_CUDA(cudaMemsetAsync(full.p, 0, full.bytes, st));
     if (N > 0) {
-      k_hash_insert<<<blocks_for(N), kTPB, 0, st>>>(cb, N, dk.Current(), G->rowptr.as<int64_t>(), G->adj.as<int2>(),
+      k_hash_insert<<<blocks_for(N), kTPB, 0, st>>>(n, cb, N, sorted, G->rowptr.as<int64_t>(), G->adj.as<int2>(),
                                                     G->hoff.as<int64_t>(), G->hkey.as<int32_t>(),
-                                                    G->hval.as<int32_t>(), d_err);
+                                                    G->hval.as<int32_t>(), full.as<int32_t>());
       TS_CUDA(cudaGetLastError());
     }
     int32_t err = 0;
-    TS_CUDA(cudaMemcpyAsync(&err, d_err, sizeof(err), cudaMemcpyDeviceToHost, st));
+    TS_CUDA(cudaMemcpyAsync(&err, full.p, sizeof(err), cudaMemcpyDeviceToHost, st));
     TS_CUDA(cudaStreamSynchronize(st));
     if (err & E_HASH_FULL) {
       set_error("ts_graph_create: hash table overflow");
       return TS_ERR_DEVICE;
     }
+  }
+  if (later) {
+    temp.reset();
+    filled(G->tables);
+    if ((s = G->tables.alloc("alloc graph")) != TS_OK) return s;
+    if ((s = fill(N, nullptr)) != TS_OK) return s;
+    TS_CUDA(cudaStreamSynchronize(st));
   }
   return TS_OK;
 }

@@ -134,7 +134,10 @@ struct DevParts {
     size_t bytes = 0;
     for (auto& x : parts) bytes += pad(x.second);
     const cudaError_t e = pool_get(mem, bytes, ordered, st);
-    if (e != cudaSuccess) return cuda_fail(e, what);
+    if (e != cudaSuccess) {
+      parts.clear();
+      return cuda_fail(e, what);
+    }
     unsigned char* p = static_cast<unsigned char*>(mem.p);
     for (auto& x : parts) {
       x.first->p = p;
@@ -161,7 +164,7 @@ struct ts_graph {
   int64_t wpr = 0;
   int64_t hash_slots = 0;
   tsb::Pool* pool = nullptr;  // entered by the graph
-  tsb::DevParts mem, tables;  // what is known before the sort; the hash tables
+  tsb::DevParts mem, tables;  // what is known before the sort; the hash tables, or what had to wait for room
   tsb::DevPart rowptr, adj, bits, hoff, hkey, hval, rev, wrange;
   // Host copy of the CSR row pointers/degrees (for footprint planning and the
   // solver's staging budgets); small: n+1 int64.
