@@ -20,6 +20,7 @@
 
 #include "cand.h"
 #include "sweep.cuh"
+#include "topup.h"
 #include "ts_host.h"
 
 namespace tsb {
@@ -930,8 +931,8 @@ ts_status enqueue_launches(ts_solver* s, int64_t iters) {
 // Waits for the admitted batch; tops it up when exact passes consumed launches.
 ts_status finish_batch(ts_solver* s) {
   ts_status rc;
-  int64_t last = s->h_st->iter;
-  for (int guard = 0; guard < 1 << 20; guard++) {
+  TopUp round(s->h_st->iter);
+  for (;;) {
     if ((rc = read_state(s)) != TS_OK) return rc;
     if (s->h_st->err) {
       s->matrix = false;
@@ -939,15 +940,14 @@ ts_status finish_batch(ts_solver* s) {
       return TS_ERR_DEVICE;
     }
     if (s->h_st->done || s->h_st->iter >= s->admitted_target) return TS_OK;
+    if (!round.advance(s->h_st->iter)) break;
     const int64_t left = s->admitted_target - s->h_st->iter;
     if (!s->cand.cs) {
       if ((rc = enqueue_sweeps(s, left + 1, false)) != TS_OK) return rc;
       continue;
     }
-    // The candidate pass stopped: some sweeps, then it tries again.  Stops in
-    // quick succession (ties everywhere) double the sweeps between tries.
-    s->backoff = s->h_st->iter - last > 4 * s->backoff ? 1 : std::min<int64_t>(2 * s->backoff, 4096);
-    last = s->h_st->iter;
+    // The candidate pass stopped: some sweeps, then it tries again.
+    s->backoff = round.sweeps_after(s->backoff);
     const int64_t sweeps = std::min<int64_t>(left, s->backoff);
     if ((rc = enqueue_sweeps(s, sweeps, false)) != TS_OK) return rc;
     if ((rc = enqueue_launches(s, left - sweeps)) != TS_OK) return rc;
