@@ -1,8 +1,24 @@
-// topup.h -- completing a batch of iterations after its first launches.
+// topup.h -- sweeps between two tries of the candidate pass, and the rounds that
+// complete a batch of iterations after its first launches.
 #pragma once
 #include <cstdint>
 
+#ifdef __CUDACC__
+#define TS_HOST_DEVICE __host__ __device__
+#else
+#define TS_HOST_DEVICE
+#endif
+
 namespace tsb {
+
+// Sweeps until the next try of the candidate pass, when the last try came after
+// `sweeps` of them and `gained` iterations have been made since: stops in
+// quick succession (ties everywhere) double them.
+constexpr int64_t kMaxSweeps = 4096;
+TS_HOST_DEVICE inline int64_t sweeps_after(int64_t sweeps, int64_t gained) {
+  if (gained > 4 * sweeps) return 1;
+  return 2 * sweeps < kMaxSweeps ? 2 * sweeps : kMaxSweeps;
+}
 
 // The candidate pass hands single iterations to the sweeps, any number of them
 // in a long batch: each time the host sees how far the search came, launches
@@ -10,7 +26,6 @@ namespace tsb {
 // nothing mean that the search is stuck.
 struct TopUp {
   static constexpr int kStuckRounds = 1 << 20;
-  static constexpr int64_t kMaxSweeps = 4096;
 
   explicit TopUp(int64_t iter) : last(iter) {}
   // A round that begins at iteration `iter`; false: the search is stuck.
@@ -20,12 +35,7 @@ struct TopUp {
     stuck = gained > 0 ? 0 : stuck + 1;
     return stuck < kStuckRounds;
   }
-  // Sweeps until the next try, after `sweeps` of them the last time: stops in
-  // quick succession (ties everywhere) double them.
-  int64_t sweeps_after(int64_t sweeps) const {
-    if (gained > 4 * sweeps) return 1;
-    return 2 * sweeps < kMaxSweeps ? 2 * sweeps : kMaxSweeps;
-  }
+  int64_t sweeps_after(int64_t sweeps) const { return tsb::sweeps_after(sweeps, gained); }
 
   int64_t last, gained = 0;
   int stuck = 0;

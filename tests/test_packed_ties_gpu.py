@@ -1,0 +1,66 @@
+"""Packed solves (batched form) of searches that the candidate pass leaves to the
+sweeps: the same results as the oracle's on every cluster size, and no slower
+than with the sweep pinned."""
+import time
+
+import numpy as np
+import pytest
+
+import ts_b200 as T
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+FIXED = T.TENURE_FIXED
+
+
+def all_but_a_matching(n):
+    """Every pair but (0, 1), (2, 3), ... joined by weight 1: ties everywhere."""
+    u, v = np.triu_indices(n, 1)
+    keep = (u // 2) != (v // 2)
+    return u[keep].astype(np.int32), v[keep].astype(np.int32), np.ones(int(keep.sum()), np.int32)
+
+
+@pytest.mark.parametrize("kind", T.STRUCT_NAMES)
+@pytest.mark.parametrize("problem", [T.PROBLEM_MDP, T.PROBLEM_MAXBS])
+def test_tied_searches_on_every_cluster_size(gpu, problem, kind):
+    n = 260
+    drop = problem == T.PROBLEM_MDP
+    u, v, w = all_but_a_matching(n)
+    w[::97] = 3  # a few pairs stand out: the pass settles some iterations
+    kw = dict(m=60 if drop else 0, max_iter=150, tenure_policy=FIXED, tenure=9, piter=20, gamma=12, seed=4)
+    o = O.run(O.Graph(n, u, v, w, drop_self_loops=drop), O.MDP if drop else O.MAXBS, threads=0, **kw)
+    g = T.Graph(n, u, v, w, kind, drop_self_loops=drop)
+    got = T.batch_solve([T.BatchJobSpec(g, problem, cluster=cs, **kw) for cs in (0, 1, 2, 4, 8)])
+    for r in got:
+        assert (r.iterations, r.evaluations, r.cur, r.best, r.best_true, r.stopped, r.device_error) == \
+               (o.iterations, o.evaluations, o.cur, o.best, o.best_true, o.stopped, 0)
+        np.testing.assert_array_equal(r.best_sol, got[0].best_sol)
+    g.close()
+
+
+@pytest.mark.parametrize("problem", [T.PROBLEM_MDP, T.PROBLEM_MAXBS])
+def test_failed_tries_do_not_add_up(gpu, problem):
+    """Where every iteration is left to the sweep, tries get rare (Max Bisection:
+    a try at every iteration took 1.25 times the sweeps' time)."""
+    n = 150
+    u, v, w = all_but_a_matching(n)
+    g = T.Graph(n, u, v, w, "csr", drop_self_loops=problem == T.PROBLEM_MDP)
+
+    def batch_time(sweep):
+        b = T.Batch([T.BatchJobSpec(g, problem, m=30, max_iter=2000, tenure_policy=FIXED, tenure=8, seed=k + 1, cluster=1,
+                                    piter=10 ** 6, sweep=sweep) for k in range(40)])
+        best = 1e9
+        for _ in range(5):
+            t = time.perf_counter()
+            b.launch()
+            b.sync()
+            best = min(best, time.perf_counter() - t)
+        out = [(r.cur, r.best) for r in b.results()]
+        b.close()
+        return best, out
+
+    pinned, want = min((batch_time(s) for s in (T.PASS_TILE, T.PASS_ROWS)), key=lambda x: x[0])
+    auto, got = batch_time(T.PASS_AUTO)
+    g.close()
+    assert got == want
+    assert auto < 1.15 * pinned, (auto, pinned)

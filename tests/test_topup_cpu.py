@@ -27,8 +27,8 @@ int main() {
   for (int k = 0; k < 30; k++, iter += sweeps) {
     if (!d.advance(iter)) return 3;
     sweeps = d.sweeps_after(sweeps);
-    const int64_t want = k < 12 ? int64_t(2) << k : TopUp::kMaxSweeps;
-    if (sweeps != (want < TopUp::kMaxSweeps ? want : TopUp::kMaxSweeps)) return 4;
+    const int64_t want = k < 12 ? int64_t(2) << k : tsb::kMaxSweeps;
+    if (sweeps != (want < tsb::kMaxSweeps ? want : tsb::kMaxSweeps)) return 4;
   }
   // nothing advances: an end, and one iteration starts the count again
   TopUp s(7);
