@@ -400,9 +400,10 @@ ts_status plan_group_st(Group& G, std::vector<BatchJobDev>& table, int64_t budge
   }
 }
 
-// CTAs per solve of a pinned sweep when the job asks for "auto": a solve whose share of the
-// batch's work would outlast the rest on one CTA is spread over a cluster, so
-// the batch does not end on one long solve.
+// CTAs per solve that sweeps (pinned, or without the candidate pass) when the
+// job asks for "auto": a solve whose share of the batch's work would outlast the
+// rest on one CTA is spread over a cluster, so the batch does not end on one
+// long solve.
 int32_t auto_cluster(double work, double total, int sms) {
   const double share = work * (2.0 * sms) / std::max(1.0, total);
   if (share < 0.5) return 1;
@@ -498,8 +499,12 @@ ts_status ts_batch_create(const ts_batch_job* jobs, int32_t count, const ts_batc
   int64_t ctas = 0;
   for (auto& H : hj) {
     if (!H.cluster) {
-      H.cluster = H.p.pass == TS_PASS_AUTO ? cand_cluster(H.n) : auto_cluster(H.work, total, sms);
-      if (H.p.pass == TS_PASS_AUTO && H.p.problem == TS_PROBLEM_MAXBS && H.n > 2048 && H.cluster < 4) widen.push_back(&H);
+      H.cluster = cand_cluster(H.g, H.p.problem, H.m, H.wide, H.p.pass);
+      const bool cand = H.cluster > 0;
+      // a tenure that makes a whole side tabu leaves the iterations to the sweeps
+      const bool sides_tabu = H.p.problem == TS_PROBLEM_MAXBS && H.p.tenure_policy == TS_TENURE_FIXED && H.p.tenure >= H.m;
+      if (!cand || sides_tabu) H.cluster = std::max(H.cluster, auto_cluster(H.work, total, sms));
+      if (cand && H.p.problem == TS_PROBLEM_MAXBS && H.n > 2048 && H.cluster < 4) widen.push_back(&H);
     }
     ctas += H.cluster;
   }

@@ -134,8 +134,16 @@ CandPlan cand_slices(const ts_graph* g, int32_t problem, int32_t m, bool wide, i
   return p;
 }
 
+// In a complete graph of equal weights all vertices of a side are alike: every
+// pair ties and the pass never settles an iteration.  Its shared memory would
+// only keep other CTAs of the sweeps off the SM (200 MDP solves of n = 600: 92
+// ms without it, 175 with it).
+static bool every_pair_ties(const ts_graph* g) {
+  return g->entries == (int64_t)g->n * (g->n - 1) && g->max_wdeg == (g->n - 1) * g->max_abs_w;
+}
+
 CandPlan cand_persist(const ts_graph* g, int32_t problem, int32_t m, bool wide, int32_t pass, int cs) {
-  if (pass != TS_PASS_AUTO) return CandPlan{};
+  if (pass != TS_PASS_AUTO || every_pair_ties(g)) return CandPlan{};
   CandPlan p = cand_slices(g, problem, m, wide, cs, kCandPersistSmem);
   if (!p.cs) return CandPlan{};
   // The cluster's own sweep is the alternative: it passes eight pairs or more
@@ -148,8 +156,12 @@ CandPlan cand_persist(const ts_graph* g, int32_t problem, int32_t m, bool wide, 
 // CTA against four took 2.7 against 3.4 us (MDP, n = 5,000), 12.9 against 10.0
 // us (Max Bisection, n = 5,000) and 22 against 11.7 us (n = 12,000) -- less
 // than twice as fast on four times the SMs.  Larger solves need the other
-// CTAs' shared memory.
-int cand_cluster(int32_t n) { return n <= 6144 ? 1 : (n <= 16384 ? 2 : 4); }
+// CTAs' shared memory: as many as hold the state, up to eight.
+int cand_cluster(const ts_graph* g, int32_t problem, int32_t m, bool wide, int32_t pass) {
+  for (int cs = g->n <= 6144 ? 1 : (g->n <= 16384 ? 2 : 4); cs <= 8; cs *= 2)
+    if (cand_persist(g, problem, m, wide, pass, cs).cs) return cs;
+  return 0;
+}
 
 CandPlan cand_plan(const ts_graph* g, int32_t problem, int32_t m, bool wide) {
   // Max Bisection spends most of an iteration on candidate rows, which more

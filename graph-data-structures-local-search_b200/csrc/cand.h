@@ -22,10 +22,12 @@ struct CandPlan {
 // Slices for a given cluster size within `limit` bytes of shared memory.
 CandPlan cand_slices(const ts_graph* g, int32_t problem, int32_t m, bool wide, int cs, size_t limit);
 // The same for a persistent (batched, served) solve; cs 0 when the pass does
-// not apply: a pinned sweep, or a state too large for the cluster.
+// not apply: a pinned sweep, a graph on which every pair ties, or a state too
+// large for the cluster.
 CandPlan cand_persist(const ts_graph* g, int32_t problem, int32_t m, bool wide, int32_t pass, int cs);
-// Cluster size of a persistent solve whose caller leaves it open.
-int cand_cluster(int32_t n);
+// Cluster size of a persistent solve whose caller leaves it open; 0 when no
+// cluster has the pass.
+int cand_cluster(const ts_graph* g, int32_t problem, int32_t m, bool wide, int32_t pass);
 // The plain form's choice of cluster size.
 CandPlan cand_plan(const ts_graph* g, int32_t problem, int32_t m, bool wide);
 // `solver` points to a DevSolver<KeyT> (KeyT by `wide`).

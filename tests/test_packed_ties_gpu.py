@@ -64,3 +64,51 @@ def test_failed_tries_do_not_add_up(gpu, problem):
     g.close()
     assert got == want
     assert auto < 1.15 * pinned, (auto, pinned)
+
+
+def complete(n):
+    u, v = (x.astype(np.int32) for x in np.triu_indices(n, 1))
+    return u, v, np.ones(len(u), np.int32)
+
+
+def sparse(n, deg, seed):
+    rng = np.random.default_rng(seed)
+    a, b = rng.integers(0, n, (2, int(n * deg / 2)))
+    key = np.unique(np.minimum(a, b)[a != b] * n + np.maximum(a, b)[a != b])
+    return (key // n).astype(np.int32), (key % n).astype(np.int32), rng.integers(1, 1001, len(key)).astype(np.int32)
+
+
+@pytest.mark.parametrize("case", ["complete", "complete, many", "sides tabu", "too large"])
+def test_open_cluster_of_swept_solves(gpu, case):
+    """A batch that leaves the cluster sizes open gives solves that sweep as many
+    CTAs as the pinned sweep gets, so it is not slower."""
+    problem, count, kw = T.PROBLEM_MAXBS, 4, dict(max_iter=60, tenure=10)
+    if case == "complete":
+        n, edges = 1000, complete(1000)
+    elif case == "complete, many":
+        problem, count, kw = T.PROBLEM_MDP, 200, dict(m=80, max_iter=60, tenure=8)
+        n, edges = 500, complete(500)
+    elif case == "sides tabu":
+        n, edges, kw = 1500, sparse(1500, 12, 1), dict(max_iter=1200, tenure=1000, piter=10 ** 6)
+    else:
+        problem, count, kw = T.PROBLEM_MDP, 2, dict(m=300, max_iter=20, tenure=20)
+        n, edges = 330_000, sparse(330_000, 8, 2)
+    g = T.Graph(n, *edges, "hash", drop_self_loops=problem == T.PROBLEM_MDP)
+
+    def batch_time(sweep):
+        b = T.Batch([T.BatchJobSpec(g, problem, tenure_policy=FIXED, seed=k + 1, sweep=sweep, **kw) for k in range(count)])
+        best = 1e9
+        for _ in range(4):
+            t = time.perf_counter()
+            b.launch()
+            b.sync()
+            best = min(best, time.perf_counter() - t)
+        out = [(r.cur, r.best, r.iterations) for r in b.results()]
+        b.close()
+        return best, out
+
+    pinned, want = min((batch_time(s) for s in (T.PASS_TILE, T.PASS_ROWS)), key=lambda x: x[0])
+    auto, got = batch_time(T.PASS_AUTO)
+    g.close()
+    assert got == want
+    assert auto < 1.15 * pinned, (auto, pinned)
