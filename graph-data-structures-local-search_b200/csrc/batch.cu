@@ -5,7 +5,8 @@
 // drivers call that loop again and again for restarts and offspring (OBMA
 // :754-903,1146-1208; MACUT src/maxbisection/GPU-MAXBS-CSR.cu:523-577,679-732).
 //
-// Here solves are grouped by (problem, structure, key width, CTAs per solve)
+// Here solves are grouped by (problem, structure, key width, CTAs per solve,
+// sweeps alone or with the candidate pass)
 // and each group is ONE persistent launch.  A thread-block cluster of 1-8 CTAs
 // owns one slot of solver memory in HBM: it pulls a solve from the group's job
 // list (atomic ticket), its leader CTA builds the start state, then the cluster
@@ -114,7 +115,7 @@ __device__ DevSolver<KeyT> slot_solver(const BatchJobDev& J, const SlotPool<KeyT
   return s;
 }
 
-template <int PROB, int ST, class KeyT>
+template <int PROB, int ST, class KeyT, bool CAND>
 __global__ void __launch_bounds__((TpbOf<ST, true>::v))
 batch_kernel(const BatchJobDev* __restrict__ jobs, int njobs, BatchResultDev* __restrict__ out,
              int32_t* __restrict__ best_out, const SlotPool<KeyT> pool, unsigned int* next_job) {
@@ -125,7 +126,7 @@ batch_kernel(const BatchJobDev* __restrict__ jobs, int njobs, BatchResultDev* __
   __shared__ TailShared sh;
   __shared__ int s_job;
   __shared__ CtaRec s_rec;
-  __shared__ CandShared<KeyT> s_cand;
+  __shared__ CandSharedIf<CAND, KeyT> s_cand;
   __shared__ long long sc[kMaxTPB / 32];
   __shared__ int32_t s_cnt[kMaxTPB];
   for (;;) {
@@ -142,7 +143,7 @@ batch_kernel(const BatchJobDev* __restrict__ jobs, int njobs, BatchResultDev* __
       __threadfence();
     }
     cl.sync();
-    cluster_iterate<PROB, ST, KeyT>(g, s, J.max_iter, cl, sh, s_rec, s_cand);
+    cluster_iterate<PROB, ST, KeyT, CAND>(g, s, J.max_iter, cl, sh, s_rec, s_cand);
     if (rank == 0) slot_finish<PROB, KeyT>(g, s, out + J.orig, best_out + J.sol_off, sc);
   }
 }
@@ -152,7 +153,7 @@ struct HostJob {
   const ts_graph* g;
   ts_params p;
   int32_t n, m, num_pert, cluster;
-  bool wide;
+  bool wide, cand;  // cand: has the candidate pass on its cluster
   int32_t kind;
   long long events;
   double work;
@@ -206,7 +207,7 @@ using Launcher = std::function<cudaError_t(cudaStream_t, const BatchJobDev*, Bat
 
 struct Group {
   int32_t problem = 0, kind = 0, cluster = 1;
-  bool wide = false;
+  bool wide = false, cand = false;
   std::vector<HostJob*> jobs;
   long long job_off = 0;  // first entry in the device job table
   double work = 0;
@@ -249,7 +250,7 @@ namespace tsb {
 namespace {
 
 // Geometry of every job of the group, slot pool within the budget, launcher.
-template <int PROB, int ST, class KeyT>
+template <int PROB, int ST, class KeyT, bool CAND>
 ts_status plan_group(Group& G, std::vector<BatchJobDev>& table, int64_t budget_bytes,
                      int32_t max_slots, int sms) {
   constexpr int R = Rows<ST>::R;
@@ -273,8 +274,8 @@ ts_status plan_group(Group& G, std::vector<BatchJobDev>& table, int64_t budget_b
     J.chunk_cols = tg.chunk_cols;
     J.n_chunks = tg.n_chunks;
     J.stage_bytes = tg.stage_bytes;
-    const CandPlan cp = cand_persist(H.g, PROB, H.m, sizeof(KeyT) == 8, H.p.pass, cs);
-    J.cand_rpc = cp.cs ? cp.rpc : 0;
+    const CandPlan cp = CAND ? cand_persist(H.g, PROB, H.m, sizeof(KeyT) == 8, H.p.pass, cs) : CandPlan{};
+    J.cand_rpc = cp.rpc;
     J.cand_cpc = cp.cpc;
     J.cand_vpc = cp.vpc;
     J.cand_list = cp.list;
@@ -282,7 +283,7 @@ ts_status plan_group(Group& G, std::vector<BatchJobDev>& table, int64_t budget_b
     J.cand_fav = cp.fav;
     J.cand_plus = cp.plus;
     J.cand_pairs = cp.pairs;
-    smem = std::max(smem, std::max(tg.smem, cp.cs ? cp.smem : (size_t)0));
+    smem = std::max(smem, std::max(tg.smem, cp.smem));
     max_m = std::max<long long>(max_m, H.m);
     max_n = std::max<long long>(max_n, H.n);
     max_ldc = std::max<long long>(max_ldc, ldc);
@@ -293,7 +294,7 @@ ts_status plan_group(Group& G, std::vector<BatchJobDev>& table, int64_t budget_b
     log_cap = std::max(log_cap, lc);
   }
   G.smem = smem;
-  auto kern = batch_kernel<PROB, ST, KeyT>;
+  auto kern = batch_kernel<PROB, ST, KeyT, CAND>;
   TS_CUDA(allow_dyn_smem(reinterpret_cast<const void*>(kern), smem));
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -387,17 +388,22 @@ ts_status plan_group(Group& G, std::vector<BatchJobDev>& table, int64_t budget_b
   return TS_OK;
 }
 
-template <int PROB, class KeyT>
+template <int PROB, class KeyT, bool CAND>
 ts_status plan_group_st(Group& G, std::vector<BatchJobDev>& table, int64_t budget, int32_t max_slots,
                         int sms) {
   switch (G.kind) {
-    case S_CSR: return plan_group<PROB, S_CSR, KeyT>(G, table, budget, max_slots, sms);
-    case S_HASH: return plan_group<PROB, S_HASH, KeyT>(G, table, budget, max_slots, sms);
-    case S_WSWAP: return plan_group<PROB, S_WSWAP, KeyT>(G, table, budget, max_slots, sms);
-    case S_BITSET: return plan_group<PROB, S_BITSET, KeyT>(G, table, budget, max_slots, sms);
-    case S_BB: return plan_group<PROB, S_BB, KeyT>(G, table, budget, max_slots, sms);
-    default: return plan_group<PROB, S_BITSET_BB, KeyT>(G, table, budget, max_slots, sms);
+    case S_CSR: return plan_group<PROB, S_CSR, KeyT, CAND>(G, table, budget, max_slots, sms);
+    case S_HASH: return plan_group<PROB, S_HASH, KeyT, CAND>(G, table, budget, max_slots, sms);
+    case S_WSWAP: return plan_group<PROB, S_WSWAP, KeyT, CAND>(G, table, budget, max_slots, sms);
+    case S_BITSET: return plan_group<PROB, S_BITSET, KeyT, CAND>(G, table, budget, max_slots, sms);
+    case S_BB: return plan_group<PROB, S_BB, KeyT, CAND>(G, table, budget, max_slots, sms);
+    default: return plan_group<PROB, S_BITSET_BB, KeyT, CAND>(G, table, budget, max_slots, sms);
   }
+}
+template <int PROB, class KeyT>
+ts_status plan_group_cand(Group& G, std::vector<BatchJobDev>& table, int64_t budget, int32_t max_slots, int sms) {
+  return G.cand ? plan_group_st<PROB, KeyT, true>(G, table, budget, max_slots, sms)
+                : plan_group_st<PROB, KeyT, false>(G, table, budget, max_slots, sms);
 }
 
 // CTAs per solve that sweeps (pinned, or without the candidate pass) when the
@@ -489,7 +495,8 @@ ts_status ts_batch_create(const ts_batch_job* jobs, int32_t count, const ts_batc
     TS_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
     b->own_stream = true;
   }
-  // groups by (problem, structure, key width, CTAs per solve); largest solves first
+  // groups by (problem, structure, key width, CTAs per solve, sweeps alone or
+  // with the candidate pass); largest solves first
   double total = 0;
   for (auto& H : hj) total += H.work;
   // Open cluster sizes.  Where the batch leaves SMs idle, the bisections that
@@ -516,9 +523,10 @@ ts_status ts_batch_create(const ts_batch_job* jobs, int32_t count, const ts_batc
   }
   for (auto& H : hj) {
     const int32_t cs = H.cluster;
+    H.cand = cand_persist(H.g, H.p.problem, H.m, H.wide, H.p.pass, cs).cs > 0;
     Group* G = nullptr;
     for (auto& x : b->groups)
-      if (x.problem == H.p.problem && x.kind == H.kind && x.wide == H.wide && x.cluster == cs) G = &x;
+      if (x.problem == H.p.problem && x.kind == H.kind && x.wide == H.wide && x.cluster == cs && x.cand == H.cand) G = &x;
     if (!G) {
       b->groups.emplace_back();
       G = &b->groups.back();
@@ -526,6 +534,7 @@ ts_status ts_batch_create(const ts_batch_job* jobs, int32_t count, const ts_batc
       G->kind = H.kind;
       G->wide = H.wide;
       G->cluster = cs;
+      G->cand = H.cand;
     }
     G->jobs.push_back(&H);
     G->work += H.work;
@@ -595,11 +604,11 @@ ts_status ts_batch_create(const ts_batch_job* jobs, int32_t count, const ts_batc
   for (auto& G : b->groups) {
     const int64_t gb = (int64_t)((double)budget * G.work / std::max(1.0, total));
     if (G.problem == P_MDP)
-      rc = G.wide ? plan_group_st<P_MDP, long long>(G, table, gb, o.max_slots, sms)
-                  : plan_group_st<P_MDP, int32_t>(G, table, gb, o.max_slots, sms);
+      rc = G.wide ? plan_group_cand<P_MDP, long long>(G, table, gb, o.max_slots, sms)
+                  : plan_group_cand<P_MDP, int32_t>(G, table, gb, o.max_slots, sms);
     else
-      rc = G.wide ? plan_group_st<P_MAXBS, long long>(G, table, gb, o.max_slots, sms)
-                  : plan_group_st<P_MAXBS, int32_t>(G, table, gb, o.max_slots, sms);
+      rc = G.wide ? plan_group_cand<P_MAXBS, long long>(G, table, gb, o.max_slots, sms)
+                  : plan_group_cand<P_MAXBS, int32_t>(G, table, gb, o.max_slots, sms);
     if (rc != TS_OK) return rc;
     b->info.slots += G.slots;
     b->info.slot_bytes += (int64_t)G.pool->bytes;

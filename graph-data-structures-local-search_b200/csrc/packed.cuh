@@ -190,6 +190,13 @@ __device__ void slot_finish(const DevGraph& g, const DevSolver<KeyT>& s, BatchRe
   __syncthreads();
 }
 
+// Shared memory of the candidate pass in kernels that have it.
+template <bool CAND, class KeyT>
+struct CandSharedIf {
+  CandShared<KeyT> v;
+};
+template <class KeyT>
+struct CandSharedIf<false, KeyT> {};
 
 // Runs a solve's iterations up to `stop_at` with the CTAs of the calling
 // cluster: the candidate pass where the solve has it, else (and for the
@@ -199,20 +206,27 @@ __device__ void slot_finish(const DevGraph& g, const DevSolver<KeyT>& s, BatchRe
 // stops in quick succession double the sweeps between tries (bisection of n =
 // 150 with ties everywhere, 2,000 iterations: 149 ms with a try at each, 120.5
 // with fewer, 119 with the sweep pinned).  Every CTA of the cluster calls it.
-template <int PROB, int ST, class KeyT>
+//
+// CAND: the solve has the candidate pass.  Kernels for solves without it
+// (pinned sweeps above all) are compiled without it: its registers and its code
+// beside the sweep's cost them up to two thirds (64 MDP solves of n = 2,000 on
+// the tile pass 23.5 -> 38.6 ms, 300 bisections 112 -> 140, on the per-row pass
+// 302 -> 387).
+template <int PROB, int ST, class KeyT, bool CAND>
 __device__ void cluster_iterate(const DevGraph& g, const DevSolver<KeyT>& s, long long stop_at,
                                 cooperative_groups::cluster_group& cl, TailShared& sh, CtaRec& s_rec,
-                                CandShared<KeyT>& s_cand) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+                                CandSharedIf<CAND, KeyT>& s_cand) {
+  [[maybe_unused]] extern __shared__ __align__(16) unsigned char smem_raw[];
   const unsigned rank = cl.block_rank(), cs = cl.num_blocks();
   const int tid = threadIdx.x;
   const int ntiles = s.n_row_blocks * s.n_chunks;
   const DevState* st = s.st;
-  long long last = __ldcg(&st->iter);  // at the last try of the candidate pass
-  int32_t sweeps = 1, wait = 0;        // between tries; left until the next
+  long long last = CAND ? __ldcg(&st->iter) : 0;  // at the last try of the candidate pass
+  int32_t sweeps = 1, wait = 0;                   // between tries; left until the next
   for (;;) {
-    const bool tried = s.cand_rpc > 0 && wait == 0;
-    if (tried && cand_run<PROB, ST, KeyT>(g, s, stop_at, LLONG_MAX, cl, s_cand, smem_raw) == kCandEnd) break;
+    const bool tried = CAND && wait == 0;
+    if constexpr (CAND)
+      if (tried && cand_run<PROB, ST, KeyT>(g, s, stop_at, LLONG_MAX, cl, s_cand.v, smem_raw) == kCandEnd) break;
     // every CTA reads the same state: the leader wrote it before the last barrier
     const long long it = __ldcg(&st->iter);
     if (__ldcg(&st->done) || it >= stop_at) break;

@@ -53,14 +53,14 @@ struct ServeJobDev {
 };
 
 // One cluster per job; the job runs until stop_at, its end or max_iter.
-template <int PROB, int ST, class KeyT>
+template <int PROB, int ST, class KeyT, bool CAND>
 __global__ void __launch_bounds__((TpbOf<ST, true>::v))
 serve_kernel(const ServeJobDev<KeyT>* __restrict__ jobs) {
   cg::cluster_group cl = cg::this_cluster();
   const unsigned rank = cl.block_rank(), cs = cl.num_blocks();
   __shared__ TailShared sh;
   __shared__ CtaRec s_rec;
-  __shared__ CandShared<KeyT> s_cand;
+  __shared__ CandSharedIf<CAND, KeyT> s_cand;
   __shared__ long long sc[kMaxTPB / 32];
   __shared__ int32_t s_cnt[kMaxTPB];
   const ServeJobDev<KeyT> J = jobs[blockIdx.x / cs];
@@ -69,7 +69,7 @@ serve_kernel(const ServeJobDev<KeyT>* __restrict__ jobs) {
     __threadfence();
   }
   cl.sync();
-  cluster_iterate<PROB, ST, KeyT>(J.g, J.s, J.stop_at < J.max_iter ? J.stop_at : J.max_iter, cl, sh, s_rec, s_cand);
+  cluster_iterate<PROB, ST, KeyT, CAND>(J.g, J.s, J.stop_at < J.max_iter ? J.stop_at : J.max_iter, cl, sh, s_rec, s_cand);
   if (rank == 0) {
     const DevState* st = J.s.st;
     if (__ldcg(&st->done) || __ldcg(&st->iter) >= J.max_iter)
@@ -77,9 +77,9 @@ serve_kernel(const ServeJobDev<KeyT>* __restrict__ jobs) {
   }
 }
 
-template <int PROB, int ST, class KeyT>
+template <int PROB, int ST, class KeyT, bool CAND>
 cudaError_t launch_serve(cudaStream_t st, const void* jobs, int njobs, int cs, size_t smem) {
-  auto kern = serve_kernel<PROB, ST, KeyT>;
+  auto kern = serve_kernel<PROB, ST, KeyT, CAND>;
   cudaError_t e = allow_dyn_smem(reinterpret_cast<const void*>(kern), smem);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute a[1];
@@ -99,21 +99,26 @@ cudaError_t launch_serve(cudaStream_t st, const void* jobs, int njobs, int cs, s
 
 using ServeLauncher = cudaError_t (*)(cudaStream_t, const void*, int, int, size_t);
 
-template <int PROB, class KeyT>
+template <int PROB, class KeyT, bool CAND>
 ServeLauncher serve_launcher_st(int kind) {
   switch (kind) {
-    case S_CSR: return launch_serve<PROB, S_CSR, KeyT>;
-    case S_HASH: return launch_serve<PROB, S_HASH, KeyT>;
-    case S_WSWAP: return launch_serve<PROB, S_WSWAP, KeyT>;
-    case S_BITSET: return launch_serve<PROB, S_BITSET, KeyT>;
-    case S_BB: return launch_serve<PROB, S_BB, KeyT>;
-    default: return launch_serve<PROB, S_BITSET_BB, KeyT>;
+    case S_CSR: return launch_serve<PROB, S_CSR, KeyT, CAND>;
+    case S_HASH: return launch_serve<PROB, S_HASH, KeyT, CAND>;
+    case S_WSWAP: return launch_serve<PROB, S_WSWAP, KeyT, CAND>;
+    case S_BITSET: return launch_serve<PROB, S_BITSET, KeyT, CAND>;
+    case S_BB: return launch_serve<PROB, S_BB, KeyT, CAND>;
+    default: return launch_serve<PROB, S_BITSET_BB, KeyT, CAND>;
   }
 }
+template <int PROB, class KeyT>
+ServeLauncher serve_launcher_cand(int kind, bool cand) {
+  return cand ? serve_launcher_st<PROB, KeyT, true>(kind) : serve_launcher_st<PROB, KeyT, false>(kind);
+}
 
-ServeLauncher serve_launcher(int problem, int kind, bool wide) {
-  if (problem == P_MDP) return wide ? serve_launcher_st<P_MDP, long long>(kind) : serve_launcher_st<P_MDP, int32_t>(kind);
-  return wide ? serve_launcher_st<P_MAXBS, long long>(kind) : serve_launcher_st<P_MAXBS, int32_t>(kind);
+ServeLauncher serve_launcher(int problem, int kind, bool wide, bool cand) {
+  if (problem == P_MDP)
+    return wide ? serve_launcher_cand<P_MDP, long long>(kind, cand) : serve_launcher_cand<P_MDP, int32_t>(kind, cand);
+  return wide ? serve_launcher_cand<P_MAXBS, long long>(kind, cand) : serve_launcher_cand<P_MAXBS, int32_t>(kind, cand);
 }
 
 double now_s(std::chrono::steady_clock::time_point t0) {
@@ -131,6 +136,7 @@ struct Req {
   int64_t P = 0;
   int32_t num_pert = 1;
   bool plain = false, wide = false;
+  bool cand = false;  // packed: has the candidate pass on its cluster
   int32_t cs = 1;
   size_t smem = 16;  // packed: dynamic shared memory of one tile (tile_geometry)
   // device resources
@@ -199,7 +205,7 @@ struct ts_server {
     void* host = nullptr;
     size_t cap = 0;
   };
-  std::map<std::tuple<int, int, int, int>, Group> groups;
+  std::map<std::tuple<int, int, int, int, int>, Group> groups;
   void run();
   void admit();
   ts_status start(Req& r);
@@ -239,7 +245,8 @@ ts_status build_packed(Req& r, int32_t kind) {
   s.n_chunks = tg.n_chunks;
   s.stage_bytes = tg.stage_bytes;
   const CandPlan cp = cand_persist(r.g, r.p.problem, m, sizeof(KeyT) == 8, r.p.pass, r.cs);
-  s.cand_rpc = cp.cs ? cp.rpc : 0;
+  r.cand = cp.cs > 0;
+  s.cand_rpc = cp.rpc;
   s.cand_cpc = cp.cpc;
   s.cand_vpc = cp.vpc;
   s.cand_list = cp.list;
@@ -247,7 +254,7 @@ ts_status build_packed(Req& r, int32_t kind) {
   s.cand_fav = cp.fav;
   s.cand_plus = cp.plus;
   s.cand_pairs = cp.pairs;
-  r.smem = std::max(tg.smem, cp.cs ? cp.smem : (size_t)0);
+  r.smem = std::max(tg.smem, cp.smem);
   s.P = (int64_t)m * delta;
   const int64_t entries = r.g->entries;
   const int64_t events = r.p.problem == P_MAXBS ? r.p.max_iter / r.p.piter + 1 : 0;
@@ -468,11 +475,11 @@ void ts_server::round() {
     if (adm == 0) plain_done.push_back(&r);
   }
   // packed solves: one launch per group
-  std::map<std::tuple<int, int, int, int>, std::vector<Req*>> by_group;
+  std::map<std::tuple<int, int, int, int, int>, std::vector<Req*>> by_group;
   for (auto& rp : active) {
     Req& r = *rp;
     if (r.plain || r.ticket < 0) continue;
-    by_group[std::make_tuple(r.p.problem, r.kind, r.wide ? 1 : 0, r.cs)].push_back(&r);
+    by_group[std::make_tuple(r.p.problem, r.kind, r.wide ? 1 : 0, r.cs, r.cand ? 1 : 0)].push_back(&r);
   }
   std::vector<cudaStream_t> used;
   for (auto& kv : by_group) {
@@ -537,7 +544,7 @@ void ts_server::round() {
       r.started = true;
     }
     cudaMemcpyAsync(G.table.p, G.host, rec * js.size(), cudaMemcpyHostToDevice, G.stream);
-    ServeLauncher L = serve_launcher(std::get<0>(kv.first), std::get<1>(kv.first), wide);
+    ServeLauncher L = serve_launcher(std::get<0>(kv.first), std::get<1>(kv.first), wide, std::get<4>(kv.first) != 0);
     cudaError_t e = L(G.stream, G.table.p, (int)js.size(), std::get<3>(kv.first), smem);
     if (e != cudaSuccess) {
       ts_status rc = cuda_fail(e, "serve kernel launch");
