@@ -143,7 +143,7 @@ batch_kernel(const BatchJobDev* __restrict__ jobs, int njobs, BatchResultDev* __
       __threadfence();
     }
     cl.sync();
-    cluster_iterate<PROB, ST, KeyT, CAND>(g, s, J.max_iter, cl, sh, s_rec, s_cand);
+    cluster_iterate<PROB, ST, KeyT, CAND, false>(g, s, J.max_iter, 0, cl, sh, s_rec, s_cand);
     if (rank == 0) slot_finish<PROB, KeyT>(g, s, out + J.orig, best_out + J.sol_off, sc);
   }
 }

@@ -13,7 +13,7 @@ namespace tsb {
 struct BatchResultDev {
   long long iterations, evaluations, cur, best, best_true, perturbations;
   int32_t stopped, err;
-  int32_t complete, pad;  // complete: written when the solve has ended
+  int32_t complete, pad;  // complete: written when the solve has ended (served: until then iterations alone)
 };
 
 __device__ __forceinline__ long long block_sum(long long v, long long* sc) {
@@ -212,10 +212,14 @@ struct CandSharedIf<false, KeyT> {};
 // beside the sweep's cost them up to two thirds (64 MDP solves of n = 2,000 on
 // the tile pass 23.5 -> 38.6 ms, 300 bisections 112 -> 140, on the per-row pass
 // 302 -> 387).
-template <int PROB, int ST, class KeyT, bool CAND>
+//
+// TIMED (served): sweeps end after `budget_ns` too, wherever the search is then.
+// How many iterations of a solve the candidate pass will leave to them is not
+// known beforehand, and other requests wait for the launch.
+template <int PROB, int ST, class KeyT, bool CAND, bool TIMED>
 __device__ void cluster_iterate(const DevGraph& g, const DevSolver<KeyT>& s, long long stop_at,
-                                cooperative_groups::cluster_group& cl, TailShared& sh, CtaRec& s_rec,
-                                CandSharedIf<CAND, KeyT>& s_cand) {
+                                [[maybe_unused]] long long budget_ns, cooperative_groups::cluster_group& cl,
+                                TailShared& sh, CtaRec& s_rec, CandSharedIf<CAND, KeyT>& s_cand) {
   [[maybe_unused]] extern __shared__ __align__(16) unsigned char smem_raw[];
   const unsigned rank = cl.block_rank(), cs = cl.num_blocks();
   const int tid = threadIdx.x;
@@ -223,6 +227,8 @@ __device__ void cluster_iterate(const DevGraph& g, const DevSolver<KeyT>& s, lon
   const DevState* st = s.st;
   long long last = CAND ? __ldcg(&st->iter) : 0;  // at the last try of the candidate pass
   int32_t sweeps = 1, wait = 0;                   // between tries; left until the next
+  [[maybe_unused]] __shared__ int32_t late;       // the leader's word on the time
+  [[maybe_unused]] const long long began = TIMED ? (long long)global_ns() : 0;
   for (;;) {
     const bool tried = CAND && wait == 0;
     if constexpr (CAND)
@@ -257,9 +263,12 @@ __device__ void cluster_iterate(const DevGraph& g, const DevSolver<KeyT>& s, lon
         }
       decide_apply<PROB, ST, KeyT>(g, s, mode, k, i, sh);
       __threadfence();
+      if (TIMED && tid == 0) late = (long long)global_ns() - began > budget_ns;
     }
     cl.sync();
+    if (TIMED && *cl.map_shared_rank(&late, 0)) break;
   }
+  if (TIMED) cl.sync();  // the leader stays until its word is read
 }
 
 }  // namespace tsb

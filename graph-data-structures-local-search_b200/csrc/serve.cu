@@ -46,13 +46,15 @@ struct ServeJobDev {
   const int32_t* init;
   long long max_iter;
   long long stop_at;       // this launch runs the solve up to this iteration
+  long long budget_ns;     // and sweeps no longer than this
   int32_t need_init;
   int32_t pad;
   BatchResultDev* out;     // written when the solve ends
   int32_t* best_out;
 };
 
-// One cluster per job; the job runs until stop_at, its end or max_iter.
+// One cluster per job; the job runs until stop_at, its end or max_iter, or until
+// its sweeps have taken the launch's time.
 template <int PROB, int ST, class KeyT, bool CAND>
 __global__ void __launch_bounds__((TpbOf<ST, true>::v))
 serve_kernel(const ServeJobDev<KeyT>* __restrict__ jobs) {
@@ -69,11 +71,14 @@ serve_kernel(const ServeJobDev<KeyT>* __restrict__ jobs) {
     __threadfence();
   }
   cl.sync();
-  cluster_iterate<PROB, ST, KeyT, CAND>(J.g, J.s, J.stop_at < J.max_iter ? J.stop_at : J.max_iter, cl, sh, s_rec, s_cand);
+  cluster_iterate<PROB, ST, KeyT, CAND, true>(J.g, J.s, J.stop_at < J.max_iter ? J.stop_at : J.max_iter, J.budget_ns, cl,
+                                              sh, s_rec, s_cand);
   if (rank == 0) {
     const DevState* st = J.s.st;
     if (__ldcg(&st->done) || __ldcg(&st->iter) >= J.max_iter)
       slot_finish<PROB, KeyT>(J.g, J.s, J.out, J.best_out, sc);
+    else if (threadIdx.x == 0)
+      J.out->iterations = __ldcg(&st->iter);
   }
 }
 
@@ -149,7 +154,7 @@ struct Req {
   int32_t* d_init = nullptr;
   BatchResultDev* d_res = nullptr;
   int32_t* d_best = nullptr;
-  long long granted = 0;           // packed: iterations granted so far
+  long long at = 0;                // packed: iterations made in earlier rounds
   bool started = false;
   // plain: streams per priority level (created on first use), the current
   // level and the event that orders a move between them
@@ -337,6 +342,8 @@ ts_status ts_server::start(Req& r) {
   std::vector<int32_t>().swap(r.v);
   std::vector<int32_t>().swap(r.w);
   r.wide = 4 * r.g->max_wdeg >= (1LL << 30);
+  // a solve of few pairs may still have a state that one CTA does not hold
+  if (!r.plain) r.cs = std::max(r.cs, cand_cluster(r.g, r.p.problem, r.m, r.wide, r.p.pass));
   if (r.plain) {
     if ((rc = ts_solver_create(r.g, &r.p, &r.solver)) != TS_OK) return rc;
     return ts_solver_init(r.solver, r.initial.empty() ? nullptr : r.initial.data());
@@ -521,10 +528,10 @@ void ts_server::round() {
     for (size_t q = 0; q < js.size(); q++) {
       Req& r = *js[q];
       // seconds per iteration: the candidate pass, or the cluster's sweep
+      // (iterations that the pass leaves to it end with the round)
       const double per_cta = 5e9;
-      const double est = r.p.pass == TS_PASS_AUTO ? 6e-6 : 6e-6 + (double)r.P / (per_cta * r.cs);
+      const double est = r.cand ? 6e-6 : 6e-6 + (double)r.P / (per_cta * r.cs);
       const int64_t k = std::max<int64_t>(4, std::min<int64_t>(1 << 16, (int64_t)(round_s / est)));
-      r.granted += k;
       unsigned char* dst = static_cast<unsigned char*>(G.host) + rec * q;
       auto fill = [&](auto* J) {
         using JT = std::remove_pointer_t<decltype(J)>;
@@ -533,7 +540,8 @@ void ts_server::round() {
         std::memcpy(&J->s, r.dev_solver.data(), sizeof(J->s));
         J->init = r.d_init;
         J->max_iter = r.p.max_iter;
-        J->stop_at = r.granted;
+        J->stop_at = r.at + k;
+        J->budget_ns = (long long)(1e9 * round_s);
         J->need_init = r.started ? 0 : 1;
         J->out = r.d_res;
         J->best_out = r.d_best;
@@ -597,7 +605,10 @@ void ts_server::round() {
         r.ticket = -1;
         continue;
       }
-      if (!d.complete) continue;
+      if (!d.complete) {
+        r.at = d.iterations;
+        continue;
+      }
       ts_result res;
       std::memset(&res, 0, sizeof(res));
       res.iterations = d.iterations;

@@ -1,0 +1,59 @@
+"""How the server sizes its rounds and accounts for memory.
+
+A round lasts about ``round_ms`` whatever a request's iterations cost: requests
+whose state the candidate pass cannot hold, and searches that it leaves to the
+sweeps, must not make the others wait.
+"""
+import numpy as np
+import pytest
+
+import ts_b200 as T
+from test_serve_gpu import alone
+
+pytestmark = pytest.mark.gpu
+FIXED = T.TENURE_FIXED
+
+
+def er(n, deg, seed):
+    rng = np.random.default_rng(seed)
+    a, b = rng.integers(0, n, (2, int(n * deg / 2)))
+    key = np.unique(np.minimum(a, b)[a != b] * n + np.maximum(a, b)[a != b])
+    return (key // n).astype(np.int32), (key % n).astype(np.int32), rng.integers(1, 1001, len(key)).astype(np.int32)
+
+
+def complete(n):
+    u, v = (x.astype(np.int32) for x in np.triu_indices(n, 1))
+    return u, v, np.ones(len(u), np.int32)
+
+
+def serve(reqs, **kw):
+    srv = T.Server(**kw)
+    try:
+        tickets = [srv.submit(n, u, v, w, problem, kind=kind, **q) for n, u, v, w, problem, kind, q in reqs]
+        done = {}
+        while len(done) < len(tickets):
+            for d in srv.poll(wait_ms=50):
+                done[d.ticket] = d
+        return [done[t] for t in tickets], int(srv.stats().rounds)
+    finally:
+        srv.close()
+
+
+@pytest.mark.parametrize("case", ["no plan", "ties"])
+def test_rounds_of_swept_requests_stay_short(gpu, case):
+    """Packed requests swept at 20 us an iteration and more: 2,000 iterations
+    of them are many rounds of 2 ms."""
+    if case == "no plan":  # 280,000 vertices in the slices of four CTAs do not fit
+        n, iters = 280_000, 2000
+        u, v, w = er(n, 4, 1)
+        q = dict(m=3, max_iter=iters, tenure_policy=FIXED, tenure=1, seed=2)
+    else:  # every pair of a complete graph of equal weights ties
+        n, iters = 1200, 2000
+        u, v, w = complete(n)
+        q = dict(m=400, max_iter=iters, tenure_policy=FIXED, tenure=10, seed=2)
+    (d,), rounds = serve([(n, u, v, w, T.PROBLEM_MDP, "csr", q)], round_ms=2.0)
+    assert d.status == 0 and d.executor == "packed"
+    r = alone(n, u, v, w, T.PROBLEM_MDP, "csr", **q)
+    assert (d.result.iterations, d.result.cur, d.result.best, d.result.best_true) == (r.iterations, r.cur, r.best, r.best_true)
+    np.testing.assert_array_equal(d.result.best_sol, r.best_sol)
+    assert rounds >= 12, rounds  # at least 40 ms of sweeps; one round when each is taken for 6 us: 6
