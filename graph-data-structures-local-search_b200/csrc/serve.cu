@@ -166,19 +166,24 @@ struct Req {
   cudaEvent_t ev_a = nullptr, ev_b = nullptr;  // plain: bracket the last round's launches
 };
 
+// Device bytes a request needs at most: its graph, and beside it the builder's
+// temporaries first and the solver's state after them.
 int64_t estimate_footprint(const Req& r) {
   const int64_t n = r.n, E = (int64_t)r.u.size(), ent = 2 * E;
-  int64_t gb = 8 * (n + 1) + 8 * ent + 8 * ent;  // rowptr, adj, reverse index
-  gb += 32 * E;                                  // build temporaries
-  if (r.kind == S_BITSET || r.kind == S_BITSET_BB) gb += n * (((n + 127) / 128) * 2) * 8;
-  if (r.kind == S_HASH) gb += 8 * (n + 1) + 8 * (8 * ent + 8 * n);
+  int64_t graph = 8 * (n + 1) + 8 * (ent + 2) + 8 * n;  // rowptr, adj, weight ranges
+  if (r.kind == S_CSR) graph += 8 * ent;                // reverse index
+  if (r.kind == S_BITSET || r.kind == S_BITSET_BB) graph += n * (((n + 127) / 128) * 2) * 8;
+  if (r.kind == S_HASH) graph += 8 * (n + 1) + 8 * (8 * ent + 8 * n);
+  // keys and values to sort, two of each; the sort's scratch (0.3 bytes an
+  // edge), the hash tables' sizes
+  const int64_t build = 48 * E + E / 2 + (r.kind == S_HASH ? 8 * (n + 1) : 0);
   const int64_t m = r.m, ldc = ((n - m) + 3) & ~3LL;
-  int64_t sb = 8 * (m + ldc) * 3 + 4 * n + 4 * ent;
-  if (r.kind == S_WSWAP) sb += 4 * (m + 32) * ldc;
+  int64_t state = 8 * (m + ldc) * 3 + 4 * n + 4 * ent + 16 * n;
+  if (r.kind == S_WSWAP) state += 4 * (m + 32) * ldc;
   const int64_t events = r.p.problem == P_MAXBS ? r.p.max_iter / std::max(1, r.p.piter) + 1 : 0;
-  sb += 8 * (r.p.max_iter + 1 + (events + 1) * r.num_pert) + 8 * events * r.num_pert;
-  sb += 16 * 8 * 148;  // per-CTA records of the plain kernel
-  return gb + sb + (1 << 20);
+  state += 8 * (r.p.max_iter + 1 + (events + 1) * r.num_pert) + 8 * events * r.num_pert;
+  state += 16 * 8 * 148;  // per-CTA records of the plain kernel
+  return graph + std::max(build, state) + (1 << 20);
 }
 
 }  // namespace

@@ -57,3 +57,15 @@ def test_rounds_of_swept_requests_stay_short(gpu, case):
     assert (d.result.iterations, d.result.cur, d.result.best, d.result.best_true) == (r.iterations, r.cur, r.best, r.best_true)
     np.testing.assert_array_equal(d.result.best_sol, r.best_sol)
     assert rounds >= 12, rounds  # at least 40 ms of sweeps; one round when each is taken for 6 us: 6
+
+
+def test_footprint_counts_the_build(gpu):
+    """Keys and values to sort (two of each, 48 bytes an edge) beside the rows
+    and the reverse index."""
+    n, e = 3000, 400_000
+    rng = np.random.default_rng(3)
+    u, v = rng.integers(0, n, (2, e)).astype(np.int32)
+    w = rng.integers(1, 1001, e).astype(np.int32)
+    q = dict(m=30, max_iter=10, tenure_policy=FIXED, tenure=3, seed=1)
+    (d,), _ = serve([(n, u, v, w, T.PROBLEM_MDP, "csr", q)])
+    assert d.status == 0 and d.footprint_bytes >= (48 + 32) * e + 16 * n
