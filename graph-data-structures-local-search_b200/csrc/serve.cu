@@ -162,7 +162,8 @@ struct Req {
   int level = -1;
   cudaEvent_t moved = nullptr;
   double spi = 0;      // plain: measured seconds per iteration inside rounds (0: not yet)
-  int64_t last_k = 0;  // plain: iterations enqueued in the last round
+  int64_t advanced = 0;  // plain: iterations made in the last round
+  bool timed = false;    // plain: its launches lie between the events
   cudaEvent_t ev_a = nullptr, ev_b = nullptr;  // plain: bracket the last round's launches
 };
 
@@ -468,16 +469,11 @@ void ts_server::round() {
     const double est = r.spi > 0 ? r.spi : 12e-6 + (double)r.P / 1.5e12;
     const int64_t k = std::max<int64_t>(4, std::min<int64_t>(1 << 16, (int64_t)(target_s / est)));
     int64_t adm = 0;
-    ts_status rc = ts_solver_prepare(r.solver, k, &adm);
-    r.last_k = 0;
-    if (rc == TS_OK && adm > 0) {
-      if (!r.ev_a) cudaEventCreate(&r.ev_a);
-      if (!r.ev_b) cudaEventCreate(&r.ev_b);
-      const bool timed = r.ev_a && r.ev_b && cudaEventRecord(r.ev_a, r.g->stream) == cudaSuccess;
-      rc = ts_solver_enqueue(r.solver, adm);
-      if (rc == TS_OK && timed && cudaEventRecord(r.ev_b, r.g->stream) == cudaSuccess) r.last_k = adm;
-      cudaGetLastError();
-    }
+    if (!r.ev_a) cudaEventCreate(&r.ev_a);
+    if (!r.ev_b) cudaEventCreate(&r.ev_b);
+    ts_status rc = solver_round_begin(r.solver, k, &adm, r.ev_a);
+    r.timed = r.ev_a && r.ev_b && rc == TS_OK && adm > 0 && cudaEventRecord(r.ev_b, r.g->stream) == cudaSuccess;
+    cudaGetLastError();
     if (rc != TS_OK) {
       r.started = false;
       finish(r, rc, nullptr);
@@ -579,8 +575,7 @@ void ts_server::round() {
   for (auto& rp : active) {
     Req& r = *rp;
     if (!r.plain || r.ticket < 0) continue;
-    int64_t it = 0;
-    ts_status rc = ts_solver_sync(r.solver, &it);
+    ts_status rc = solver_round_end(r.solver, &r.advanced);
     if (rc != TS_OK) {
       finish(r, rc, nullptr);
       r.ticket = -1;
@@ -590,13 +585,13 @@ void ts_server::round() {
   last_round_s = now_s(t0) - t_round;
   for (auto& rp : active) {  // speed of each plain solve in this round (shared GPU included)
     Req& r = *rp;
-    if (!r.plain || r.ticket < 0 || r.last_k <= 0) continue;
+    if (!r.plain || r.ticket < 0 || !r.timed || r.advanced <= 0) continue;
     float ms = 0;
     if (cudaEventElapsedTime(&ms, r.ev_a, r.ev_b) != cudaSuccess || ms <= 0) {
       cudaGetLastError();
       continue;
     }
-    const double x = 1e-3 * ms / (double)r.last_k;
+    const double x = 1e-3 * ms / (double)r.advanced;
     r.spi = r.spi > 0 ? 0.5 * (r.spi + x) : x;
   }
   // packed completions

@@ -507,7 +507,10 @@ struct ts_solver {
   bool matrix = false;  // WSwap: the matrix holds the present state's weights and zeros
   int64_t admitted_target = 0;
   CandPlan cand;          // candidate pass (TS_PASS_AUTO); cs 0: sweeps only
-  int64_t backoff = 1;    // sweeps to run after the next hand-over (finish_batch)
+  int64_t backoff = 1;    // sweeps to run after the next hand-over
+  int64_t wait = 0;       // served: how many of them are left
+  int64_t round_iter = 0; // served: the iteration at which the round began
+  bool tried = false;     // served: the round ran the candidate pass
   DevState* h_st = nullptr;  // pinned mirror
 
   template <class KeyT>
@@ -928,17 +931,21 @@ ts_status enqueue_launches(ts_solver* s, int64_t iters) {
   return enqueue_sweeps(s, 1, true);
 }
 
+// Waits for what was launched and reads the state.
+ts_status settle(ts_solver* s) {
+  const ts_status rc = read_state(s);
+  if (rc != TS_OK || !s->h_st->err) return rc;
+  s->matrix = false;
+  set_error("device error word set (" + std::to_string(s->h_st->err) + ")");
+  return TS_ERR_DEVICE;
+}
+
 // Waits for the admitted batch; tops it up when exact passes consumed launches.
 ts_status finish_batch(ts_solver* s) {
   ts_status rc;
   TopUp round(s->h_st->iter);
   for (;;) {
-    if ((rc = read_state(s)) != TS_OK) return rc;
-    if (s->h_st->err) {
-      s->matrix = false;
-      set_error("device error word set (" + std::to_string(s->h_st->err) + ")");
-      return TS_ERR_DEVICE;
-    }
+    if ((rc = settle(s)) != TS_OK) return rc;
     if (s->h_st->done || s->h_st->iter >= s->admitted_target) return TS_OK;
     if (!round.advance(s->h_st->iter)) break;
     const int64_t left = s->admitted_target - s->h_st->iter;
@@ -957,6 +964,30 @@ ts_status finish_batch(ts_solver* s) {
 }
 
 }  // namespace
+
+ts_status tsb::solver_round_begin(ts_solver* s, int64_t k, int64_t* admitted, cudaEvent_t before) {
+  ts_status rc = ts_solver_prepare(s, k, admitted);
+  if (rc != TS_OK || *admitted <= 0) return rc;
+  if (before) TS_CUDA(cudaEventRecord(before, s->g->stream));
+  s->round_iter = s->h_st->iter;
+  const int64_t sweeps = s->cand.cs ? std::min(*admitted, s->wait) : *admitted;
+  s->tried = *admitted > sweeps;
+  if (s->cand.cs) s->wait -= sweeps;
+  if ((rc = enqueue_sweeps(s, sweeps, false)) != TS_OK) return rc;
+  return enqueue_launches(s, *admitted - sweeps);
+}
+
+ts_status tsb::solver_round_end(ts_solver* s, int64_t* advanced) {
+  const ts_status rc = settle(s);
+  if (rc != TS_OK) return rc;
+  *advanced = s->h_st->iter - s->round_iter;
+  if (s->tried) {
+    const bool all = s->h_st->done || s->h_st->iter >= s->admitted_target;
+    s->backoff = all ? 1 : sweeps_after(s->backoff, *advanced);
+    s->wait = all ? 0 : s->backoff;
+  }
+  return TS_OK;
+}
 
 extern "C" {
 
