@@ -141,7 +141,7 @@ struct Req {
   int64_t P = 0;
   int32_t num_pert = 1;
   bool plain = false, wide = false;
-  bool cand = false;  // packed: has the candidate pass on its cluster
+  bool cand = false;  // has the candidate pass (packed: on its cluster)
   int32_t cs = 1;
   size_t smem = 16;  // packed: dynamic shared memory of one tile (tile_geometry)
   // device resources
@@ -352,6 +352,8 @@ ts_status ts_server::start(Req& r) {
   if (!r.plain) r.cs = std::max(r.cs, cand_cluster(r.g, r.p.problem, r.m, r.wide, r.p.pass));
   if (r.plain) {
     if ((rc = ts_solver_create(r.g, &r.p, &r.solver)) != TS_OK) return rc;
+    ts_solver_info info;
+    r.cand = ts_solver_info_get(r.solver, &info) == TS_OK && info.cand_ctas > 0;
     return ts_solver_init(r.solver, r.initial.empty() ? nullptr : r.initial.data());
   }
   if (r.p.problem == P_MDP) {
@@ -466,7 +468,8 @@ void ts_server::round() {
       }
       cudaGetLastError();
     }
-    const double est = r.spi > 0 ? r.spi : 12e-6 + (double)r.P / 1.5e12;
+    // until a speed is measured: the candidate pass's, or the whole GPU's sweep
+    const double est = r.spi > 0 ? r.spi : 12e-6 + (r.cand ? 0 : (double)r.P / 1.5e12);
     const int64_t k = std::max<int64_t>(4, std::min<int64_t>(1 << 16, (int64_t)(target_s / est)));
     int64_t adm = 0;
     if (!r.ev_a) cudaEventCreate(&r.ev_a);

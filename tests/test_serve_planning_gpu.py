@@ -69,3 +69,16 @@ def test_footprint_counts_the_build(gpu):
     q = dict(m=30, max_iter=10, tenure_policy=FIXED, tenure=3, seed=1)
     (d,), _ = serve([(n, u, v, w, T.PROBLEM_MDP, "csr", q)])
     assert d.status == 0 and d.footprint_bytes >= (48 + 32) * e + 16 * n
+
+
+def test_plain_rounds_are_planned_by_the_candidate_pass(gpu):
+    """Until a speed is measured, a plain request that has the candidate pass (12
+    us an iteration) is not planned by the sweep of its 1.6e9 pairs (1.1 ms)."""
+    n = 80_000
+    u, v, w = er(n, 10, 4)
+    q = dict(max_iter=300, tenure_policy=FIXED, tenure=10, seed=3, piter=10 ** 6)
+    (d,), rounds = serve([(n, u, v, w, T.PROBLEM_MAXBS, "csr", q)], round_ms=10.0)
+    assert d.status == 0 and d.executor == "plain"
+    assert rounds <= 3, rounds  # the iterations, the result (an estimate of 1.1 ms: 9 iterations first)
+    r = alone(n, u, v, w, T.PROBLEM_MAXBS, "csr", **q)
+    assert (d.result.iterations, d.result.cur, d.result.best) == (r.iterations, r.cur, r.best)
