@@ -15,8 +15,9 @@
 // the library keeps it until the process exits.  All calls share it and it
 // keeps the last call's contents.  Calls that overlap on the GPU (from other
 // streams or host threads) race on it and decide wrongly; they read and write
-// nothing out of bounds, and leave nothing behind: each launch of a call clears
-// the other launch's ticket, so that later calls count from 0 again.
+// nothing out of bounds, and leave nothing behind: the staging ticket wraps
+// after every kNaStageCtas numbers, so it is 0 again however calls were mixed,
+// and the staging launch clears the other.
 //
 // Cost: the pairs are bounded as in the solver's candidate pass (cand.cuh).
 // One launch orders the state, takes the maxima of both sides and of the
@@ -111,7 +112,6 @@ k_na_stage(int32_t problem, int32_t n, int32_t m, long long iter, long long D, c
   __shared__ CtaRec s_top[5];
   __shared__ int32_t s_last;
   const int tid = threadIdx.x;
-  if (blockIdx.x == 0 && tid == 0) *sc.counter = 0u;
   const long long stride = (long long)gridDim.x * blockDim.x;
   long long k4[4], i4[4];
 #pragma unroll
@@ -132,7 +132,10 @@ k_na_stage(int32_t problem, int32_t n, int32_t m, long long iter, long long D, c
     for (int q = 0; q < 4; q++)
       if ((q < 2) == row && ((q & 1) || !t)) better_rec(k4[q], i4[q], y, p);
   }
-  if constexpr (!BOUNDS) return;
+  if constexpr (!BOUNDS) {
+    if (blockIdx.x == 0 && tid == 0) *sc.counter = 0u;
+    return;
+  }
   // the weights' range, as records of (max, .) and (-min, .)
   long long hi = 0, lo = 0;
   const long long E = rowptr[n];
@@ -159,7 +162,7 @@ k_na_stage(int32_t problem, int32_t n, int32_t m, long long iter, long long D, c
     sc.recs[5 * blockIdx.x + 4].key = hi;
     sc.recs[5 * blockIdx.x + 4].idx = lo;
     __threadfence();
-    s_last = atomicAdd(sc.staged, 1u) == gridDim.x - 1;
+    s_last = atomicInc(sc.staged, gridDim.x - 1) == gridDim.x - 1;
   }
   __syncthreads();
   if (!s_last) return;
@@ -223,7 +226,7 @@ k_na_stage(int32_t problem, int32_t n, int32_t m, long long iter, long long D, c
   // a seed with c*w >= 0 is the best of them
   g.need_n = (nt_ok && c1 < 0 && Am + Bm >= g.LB) || (c2 < 0 && AA + BA >= g.LT);
   *sc.goal = g;
-  *sc.staged = 0u;
+  *sc.counter = 0u;
 }
 
 // First entry of u's sorted row with neighbour v (lower_bound), else 0.
@@ -250,7 +253,6 @@ k_na_sweep(int32_t problem, int32_t n, int32_t m, long long cur, long long best,
   const int32_t delta = n - m;
   const long long P = (long long)m * delta;
   const long long D = best - cur;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *sc.staged = 0u;  // after an overlap it may have passed its mark
   long long bk = LLONG_MIN, bi = LLONG_MAX;
   if (BOUNDS && !sc.goal->all_pairs) {
     const NaGoal g = *sc.goal;
