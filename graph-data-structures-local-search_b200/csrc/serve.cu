@@ -575,14 +575,33 @@ void ts_server::round() {
     finish(*r, rc, rc == TS_OK ? &res : nullptr);
     r->ticket = -1;
   }
-  for (auto& rp : active) {
-    Req& r = *rp;
-    if (!r.plain || r.ticket < 0) continue;
-    ts_status rc = solver_round_end(r.solver, &r.advanced);
-    if (rc != TS_OK) {
-      finish(r, rc, nullptr);
-      r.ticket = -1;
+  // Plain solves whose launches have ended early go on until the round's time is
+  // up; whichever has ended is seen to first.
+  std::vector<Req*> running;
+  for (auto& rp : active)
+    if (rp->plain && rp->ticket >= 0) running.push_back(rp.get());
+  while (!running.empty()) {
+    bool idle = true;
+    for (Req*& q : running) {
+      Req& r = *q;
+      if (running.size() > 1 && cudaStreamQuery(r.g->stream) == cudaErrorNotReady) {
+        cudaGetLastError();  // no failure for the next launch to find
+        continue;
+      }
+      idle = false;
+      bool more = false;
+      const ts_status rc = solver_round_next(r.solver, now_s(t0) - t_round < target_s, &more, &r.advanced);
+      if (rc != TS_OK) {
+        finish(r, rc, nullptr);
+        r.ticket = -1;
+        more = false;
+      } else if (more) {
+        r.timed = r.timed && cudaEventRecord(r.ev_b, r.g->stream) == cudaSuccess;
+      }
+      if (!more) q = nullptr;
     }
+    running.erase(std::remove(running.begin(), running.end(), nullptr), running.end());
+    if (idle) std::this_thread::yield();
   }
   for (cudaStream_t s : used) cudaStreamSynchronize(s);
   last_round_s = now_s(t0) - t_round;

@@ -509,8 +509,9 @@ struct ts_solver {
   CandPlan cand;          // candidate pass (TS_PASS_AUTO); cs 0: sweeps only
   int64_t backoff = 1;    // sweeps to run after the next hand-over
   int64_t wait = 0;       // served: how many of them are left
-  int64_t round_iter = 0; // served: the iteration at which the round began
-  bool tried = false;     // served: the round ran the candidate pass
+  int64_t round_iter = 0; // served: the iterations at which the round
+  int64_t launch_iter = 0;  // and its last launches began
+  bool tried = false;     // served: these include the candidate pass
   DevState* h_st = nullptr;  // pinned mirror
 
   template <class KeyT>
@@ -965,28 +966,40 @@ ts_status finish_batch(ts_solver* s) {
 
 }  // namespace
 
+namespace {
+// Launches of up to `left` iterations of a served solve's round: sweeps that are
+// still due after a hand-over, then the candidate pass.
+ts_status round_launch(ts_solver* s, int64_t left) {
+  const int64_t sweeps = s->cand.cs ? std::min(left, s->wait) : left;
+  if (s->cand.cs) s->wait -= sweeps;
+  s->tried = left > sweeps;
+  s->launch_iter = s->h_st->iter;
+  const ts_status rc = enqueue_sweeps(s, sweeps, false);
+  return rc == TS_OK ? enqueue_launches(s, left - sweeps) : rc;
+}
+}  // namespace
+
 ts_status tsb::solver_round_begin(ts_solver* s, int64_t k, int64_t* admitted, cudaEvent_t before) {
-  ts_status rc = ts_solver_prepare(s, k, admitted);
+  const ts_status rc = ts_solver_prepare(s, k, admitted);
   if (rc != TS_OK || *admitted <= 0) return rc;
   if (before) TS_CUDA(cudaEventRecord(before, s->g->stream));
   s->round_iter = s->h_st->iter;
-  const int64_t sweeps = s->cand.cs ? std::min(*admitted, s->wait) : *admitted;
-  s->tried = *admitted > sweeps;
-  if (s->cand.cs) s->wait -= sweeps;
-  if ((rc = enqueue_sweeps(s, sweeps, false)) != TS_OK) return rc;
-  return enqueue_launches(s, *admitted - sweeps);
+  return round_launch(s, *admitted);
 }
 
-ts_status tsb::solver_round_end(ts_solver* s, int64_t* advanced) {
+ts_status tsb::solver_round_next(ts_solver* s, bool go_on, bool* running, int64_t* advanced) {
+  *running = false;
   const ts_status rc = settle(s);
   if (rc != TS_OK) return rc;
   *advanced = s->h_st->iter - s->round_iter;
+  const bool all = s->h_st->done || s->h_st->iter >= s->admitted_target;
   if (s->tried) {
-    const bool all = s->h_st->done || s->h_st->iter >= s->admitted_target;
-    s->backoff = all ? 1 : sweeps_after(s->backoff, *advanced);
+    s->backoff = all ? 1 : sweeps_after(s->backoff, s->h_st->iter - s->launch_iter);
     s->wait = all ? 0 : s->backoff;
   }
-  return TS_OK;
+  if (all || !go_on) return TS_OK;
+  *running = true;
+  return round_launch(s, s->admitted_target - s->h_st->iter);
 }
 
 extern "C" {

@@ -225,10 +225,11 @@ bool wswap_w16(const ts_graph* g);
 cudaError_t allow_dyn_smem(const void* fn, size_t smem);
 
 // A round of a served solve.  begin admits up to k iterations and launches them,
-// after the event `before` (null: none); end waits and says how many were made.  Unlike ts_solver_sync it does not
-// complete them: iterations that the candidate pass left to the sweeps, which
-// take many times longer, are the next rounds'.
+// after the event `before` (null: none).  next waits for the launches, says how
+// many iterations the round has made, and, where the candidate pass left one to
+// the sweeps (which take many times longer) and go_on is set, launches what comes
+// next.  Unlike ts_solver_sync it need not complete them.
 ts_status solver_round_begin(ts_solver* s, int64_t k, int64_t* admitted, cudaEvent_t before);
-ts_status solver_round_end(ts_solver* s, int64_t* advanced);
+ts_status solver_round_next(ts_solver* s, bool go_on, bool* running, int64_t* advanced);
 
 }  // namespace tsb

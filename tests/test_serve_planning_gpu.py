@@ -42,13 +42,14 @@ def serve(reqs, **kw):
 @pytest.mark.parametrize("case", ["no plan", "ties", "ties, plain"])
 def test_rounds_of_swept_requests_stay_short(gpu, case):
     """Requests swept at 20 us an iteration and more: 2,000 iterations of them
-    are many rounds of 2 ms."""
+    are many rounds of 2 ms (8,000 at 80 us: of up to 50, which a plain solve's
+    rounds may take)."""
     if case == "no plan":  # 280,000 vertices in the slices of four CTAs do not fit
         n, iters = 280_000, 2000
         u, v, w = er(n, 4, 1)
         q = dict(m=3, max_iter=iters, tenure_policy=FIXED, tenure=1, seed=2)
     else:  # every pair of a complete graph of equal weights ties
-        n, m, iters = (1200, 400, 2000) if case == "ties" else (2400, 1000, 2000)
+        n, m, iters = (1200, 400, 2000) if case == "ties" else (2400, 1000, 8000)
         u, v, w = complete(n)
         q = dict(m=m, max_iter=iters, tenure_policy=FIXED, tenure=10, seed=2)
     (d,), rounds = serve([(n, u, v, w, T.PROBLEM_MDP, "csr", q)], round_ms=2.0)
@@ -56,7 +57,7 @@ def test_rounds_of_swept_requests_stay_short(gpu, case):
     r = alone(n, u, v, w, T.PROBLEM_MDP, "csr", **q)
     assert (d.result.iterations, d.result.cur, d.result.best, d.result.best_true) == (r.iterations, r.cur, r.best, r.best_true)
     np.testing.assert_array_equal(d.result.best_sol, r.best_sol)
-    assert rounds >= 12, rounds  # at least 40 ms of sweeps; one round when each is taken for 6 us: 6
+    assert rounds >= 12, rounds  # planned at 6 us an iteration: 7; by launches that ended at once: 3
 
 
 def test_footprint_counts_the_build(gpu):
@@ -82,3 +83,20 @@ def test_plain_rounds_are_planned_by_the_candidate_pass(gpu):
     assert rounds <= 3, rounds  # the iterations, the result (an estimate of 1.1 ms: 9 iterations first)
     r = alone(n, u, v, w, T.PROBLEM_MAXBS, "csr", **q)
     assert (d.result.iterations, d.result.cur, d.result.best) == (r.iterations, r.cur, r.best)
+
+
+def test_plain_solves_go_on_after_a_hand_over(gpu):
+    """Every 60 iterations or so the candidate pass leaves one of this search (a
+    torus of weights 1 and -1) to a sweep; the solve goes on in the same round."""
+    a = b = 60
+    n = a * b
+    i = np.arange(n)
+    u = np.concatenate([i, i]).astype(np.int32)
+    v = np.concatenate([i // b * b + (i + 1) % b, (i + b) % n]).astype(np.int32)
+    w = np.where(np.random.default_rng(3).random(2 * n) < 0.5, -1, 1).astype(np.int32)
+    q = dict(max_iter=20_000, tenure_policy=FIXED, tenure=20, seed=1, piter=10 ** 6)
+    (d,), rounds = serve([(n, u, v, w, T.PROBLEM_MAXBS, "csr", q)], round_ms=5.0)
+    r = alone(n, u, v, w, T.PROBLEM_MAXBS, "csr", **q)
+    assert d.status == 0 and d.executor == "plain"
+    assert (d.result.iterations, d.result.cur, d.result.best) == (r.iterations, r.cur, r.best)
+    assert rounds <= 150, rounds
