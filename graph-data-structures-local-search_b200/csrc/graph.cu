@@ -463,8 +463,9 @@ __global__ void k_lookup(DevGraph g, int64_t count, const int32_t* __restrict__ 
 // hash tables, whose size needs the degrees, another): an allocation or a free
 // synchronises and takes 50 us to milliseconds, and a build had 12 to 20 of
 // each.  One host round trip, two for Hash.  Conflict graph, n = 100,000, 3.4M
-// edges, from host arrays: Hash 11.2 -> 5.3 ms (2.3 of them the copies), CSR
-// 8.7 -> 5.2; a million lookups 3.3 -> 1.1 ms.
+// edges, from host arrays: Hash 11.2 -> 4.2 to 5.6 ms (2.3 of them the copies;
+// the tables' plain allocation varies), CSR 8.7 -> 4.0; a million lookups 3.3 ->
+// 1.1 ms.
 // Where the device has no room for the temporaries (48 bytes an edge) beside
 // all of the graph, only what the sort fills is allocated with them, and the
 // bitmap, the reverse index or the hash tables once they are gone; these are

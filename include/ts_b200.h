@@ -254,7 +254,8 @@ ts_status ts_perturb_draws(int32_t n, uint32_t seed, int32_t gamma, int32_t init
 
 /* ---------------------------------------------------------------- batched form
  * Many independent solves (instances, restarts) in one persistent launch per
- * (problem, structure, key width, CTAs per solve) group, recorded once as a
+ * (problem, structure, key width, CTAs per solve, with or without the candidate
+ * pass) group, recorded once as a
  * CUDA graph and replayed.  Stands in for the reference's one-at-a-time
  * restart loops around tabu_search / perturbationBasedTabuSearch (OBMA
  * src/mdp/GPU-MDP-CSR.cu:754-903,1146-1208; MACUT
@@ -391,7 +392,8 @@ ts_status ts_server_destroy(ts_server* s);
  * `stream` without synchronising, in the CUDA context current on the calling
  * thread (the device's primary context if none is).  The first call in each
  * context looks the scratch address up.  All calls share the scratch, so calls that overlap on the GPU
- * (other streams or host threads) race on it.  Cost: two
+ * (other streams or host threads) race on it and decide wrongly; later calls
+ * are not affected.  Cost: two
  * launches; the rows and columns whose bounds can reach the best pair, or,
  * where no pair is allowed and below 2^20 pairs, every pair with a binary search each (roughly
  * P / 1e10 s for P = m*(n-m) pairs). */
