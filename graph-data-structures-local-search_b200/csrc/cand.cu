@@ -137,9 +137,10 @@ CandPlan cand_slices(const ts_graph* g, int32_t problem, int32_t m, bool wide, i
 // In a complete graph of equal weights all vertices of a side are alike: every
 // pair ties and the pass never settles an iteration.  Its shared memory would
 // only keep other CTAs of the sweeps off the SM (200 MDP solves of n = 600: 92
-// ms without it, 175 with it).
+// ms without it, 175 with it).  With both signs (weights of 1 and -1) the
+// contributions differ.
 static bool every_pair_ties(const ts_graph* g) {
-  return g->entries == (int64_t)g->n * (g->n - 1) && g->max_wdeg == (g->n - 1) * g->max_abs_w;
+  return !g->neg_w && g->entries == (int64_t)g->n * (g->n - 1) && g->max_wdeg == (g->n - 1) * g->max_abs_w;
 }
 
 CandPlan cand_persist(const ts_graph* g, int32_t problem, int32_t m, bool wide, int32_t pass, int cs) {
