@@ -53,6 +53,7 @@ struct BatchJobDev {
   int32_t cand_rpc, cand_cpc, cand_vpc, cand_fav, cand_list;  // candidate pass (cand_persist); 0: tiles only
   uint32_t cand_inv[3];
   long long cand_plus, cand_pairs;
+  int32_t give_up;          // candidate pass: see cluster_iterate; 0: never
   const int32_t* init;      // MDP: m ids; MaxBS: part[n]
   const long long* draws;   // MaxBS perturbation events x num_pert
   long long draw_events;
@@ -115,10 +116,13 @@ __device__ DevSolver<KeyT> slot_solver(const BatchJobDev& J, const SlotPool<KeyT
   return s;
 }
 
+// left, *left_n: solves that a launch with the candidate pass gave up, and in the
+// launch without it that follows the solves to run instead of all.
 template <int PROB, int ST, class KeyT, bool CAND>
 __global__ void __launch_bounds__((TpbOf<ST, true>::v))
 batch_kernel(const BatchJobDev* __restrict__ jobs, int njobs, BatchResultDev* __restrict__ out,
-             int32_t* __restrict__ best_out, const SlotPool<KeyT> pool, unsigned int* next_job) {
+             int32_t* __restrict__ best_out, const SlotPool<KeyT> pool, unsigned int* next_job, int32_t* left,
+             unsigned int* left_n) {
   cg::cluster_group cl = cg::this_cluster();
   const unsigned rank = cl.block_rank(), cs = cl.num_blocks();
   const long long slot = blockIdx.x / cs;
@@ -134,8 +138,8 @@ batch_kernel(const BatchJobDev* __restrict__ jobs, int njobs, BatchResultDev* __
     cl.sync();
     const int j = *cl.map_shared_rank(&s_job, 0);
     cl.sync();  // every CTA has read the leader's ticket before it changes or the leader exits
-    if (j >= njobs) return;
-    const BatchJobDev J = jobs[j];
+    if (j >= (!CAND && left ? (int)*left_n : njobs)) return;
+    const BatchJobDev J = jobs[!CAND && left ? left[j] : j];
     const DevSolver<KeyT> s = slot_solver<KeyT>(J, pool, slot, PROB);
     const DevGraph g = J.g;
     if (rank == 0) {
@@ -143,7 +147,10 @@ batch_kernel(const BatchJobDev* __restrict__ jobs, int njobs, BatchResultDev* __
       __threadfence();
     }
     cl.sync();
-    cluster_iterate<PROB, ST, KeyT, CAND, false>(g, s, J.max_iter, 0, cl, sh, s_rec, s_cand);
+    if (!cluster_iterate<PROB, ST, KeyT, CAND, false>(g, s, J.max_iter, 0, J.give_up, cl, sh, s_rec, s_cand)) {
+      if (rank == 0 && tid == 0) left[atomicAdd(left_n, 1u)] = j;
+      continue;
+    }
     if (rank == 0) slot_finish<PROB, KeyT>(g, s, out + J.orig, best_out + J.sol_off, sc);
   }
 }
@@ -153,7 +160,7 @@ struct HostJob {
   const ts_graph* g;
   ts_params p;
   int32_t n, m, num_pert, cluster;
-  bool wide, cand;  // cand: has the candidate pass on its cluster
+  bool wide, cand, open;  // cand: has the candidate pass on its cluster; open: the library chose it
   int32_t kind;
   long long events;
   double work;
@@ -203,7 +210,7 @@ bool prepare_host_job(HostJob& H, const int32_t* initial) {
 }
 
 using Launcher = std::function<cudaError_t(cudaStream_t, const BatchJobDev*, BatchResultDev*, int32_t*,
-                                           unsigned int*)>;
+                                           unsigned int*, int32_t*, unsigned int*)>;
 
 struct Group {
   int32_t problem = 0, kind = 0, cluster = 1;
@@ -215,6 +222,8 @@ struct Group {
   size_t smem = 0;
   std::unique_ptr<DevBuf> pool;
   Launcher launch;
+  std::unique_ptr<Group> swept;  // runs what the group gives up, in the same slots
+  long long left_off = 0;        // its list in ts_batch::left
 };
 
 }  // namespace
@@ -231,7 +240,7 @@ struct ts_batch {
   std::vector<cudaEvent_t> events;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  DevBuf jobs, results, best, init, draws, tickets;
+  DevBuf jobs, results, best, init, draws, tickets, left;
   std::vector<Group> groups;
   std::vector<int32_t> m_of, n_of;
   ts_batch_info info{};
@@ -252,7 +261,7 @@ namespace {
 // Geometry of every job of the group, slot pool within the budget, launcher.
 template <int PROB, int ST, class KeyT, bool CAND>
 ts_status plan_group(Group& G, std::vector<BatchJobDev>& table, int64_t budget_bytes,
-                     int32_t max_slots, int sms) {
+                     int32_t max_slots, int sms, const DevBuf* share) {
   constexpr int R = Rows<ST>::R;
   constexpr int TPB = TpbOf<ST, true>::v;
   const int cs = G.cluster;
@@ -343,12 +352,21 @@ ts_status plan_group(Group& G, std::vector<BatchJobDev>& table, int64_t budget_b
   if (max_slots > 0) slots = std::min<long long>(slots, max_slots);
   slots = std::min<long long>(slots, std::max<long long>(1, budget_bytes / (long long)per_slot));
   G.slots = slots;
-  size_t total = 0;
-  for (size_t x : slices) total += pad(x * (size_t)slots);
-  G.pool.reset(new DevBuf);
-  ts_status rc = G.pool->alloc(total, "alloc batch slots");
-  if (rc != TS_OK) return rc;
-  unsigned char* b = G.pool->as<unsigned char>();
+  auto bytes = [&](long long count) {
+    size_t total = 0;
+    for (size_t x : slices) total += pad(x * (size_t)count);
+    return total;
+  };
+  if (share) {
+    while (slots > 1 && bytes(slots) > share->bytes) slots--;
+    if (bytes(slots) > share->bytes) { set_error("ts_batch_create: shared slots too small"); return TS_ERR_UNSUPPORTED; }
+  } else {
+    G.pool.reset(new DevBuf);
+    ts_status rc = G.pool->alloc(bytes(slots), "alloc batch slots");
+    if (rc != TS_OK) return rc;
+  }
+  G.slots = slots;
+  unsigned char* b = (share ? share : G.pool.get())->as<unsigned char>();
   auto carve = [&](size_t slice) -> unsigned char* {  // one array: `slots` slices, 256 B aligned
     if (slice == 0) return nullptr;
     unsigned char* p = b;
@@ -370,7 +388,7 @@ ts_status plan_group(Group& G, std::vector<BatchJobDev>& table, int64_t budget_b
   const int njobs = (int)G.jobs.size();
   const long long off = G.job_off;
   G.launch = [=](cudaStream_t s, const BatchJobDev* djobs, BatchResultDev* dres, int32_t* dbest,
-                 unsigned int* ticket) -> cudaError_t {
+                 unsigned int* ticket, int32_t* left, unsigned int* left_n) -> cudaError_t {
     cudaLaunchAttribute a[1];
     a[0].id = cudaLaunchAttributeClusterDimension;
     a[0].val.clusterDim.x = cs;
@@ -383,27 +401,36 @@ ts_status plan_group(Group& G, std::vector<BatchJobDev>& table, int64_t budget_b
     c.stream = s;
     c.attrs = a;
     c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, kern, djobs + off, njobs, dres, dbest, pool, ticket);
+    return cudaLaunchKernelEx(&c, kern, djobs + off, njobs, dres, dbest, pool, ticket, left, left_n);
   };
   return TS_OK;
 }
 
 template <int PROB, class KeyT, bool CAND>
 ts_status plan_group_st(Group& G, std::vector<BatchJobDev>& table, int64_t budget, int32_t max_slots,
-                        int sms) {
+                        int sms, const DevBuf* share) {
   switch (G.kind) {
-    case S_CSR: return plan_group<PROB, S_CSR, KeyT, CAND>(G, table, budget, max_slots, sms);
-    case S_HASH: return plan_group<PROB, S_HASH, KeyT, CAND>(G, table, budget, max_slots, sms);
-    case S_WSWAP: return plan_group<PROB, S_WSWAP, KeyT, CAND>(G, table, budget, max_slots, sms);
-    case S_BITSET: return plan_group<PROB, S_BITSET, KeyT, CAND>(G, table, budget, max_slots, sms);
-    case S_BB: return plan_group<PROB, S_BB, KeyT, CAND>(G, table, budget, max_slots, sms);
-    default: return plan_group<PROB, S_BITSET_BB, KeyT, CAND>(G, table, budget, max_slots, sms);
+    case S_CSR: return plan_group<PROB, S_CSR, KeyT, CAND>(G, table, budget, max_slots, sms, share);
+    case S_HASH: return plan_group<PROB, S_HASH, KeyT, CAND>(G, table, budget, max_slots, sms, share);
+    case S_WSWAP: return plan_group<PROB, S_WSWAP, KeyT, CAND>(G, table, budget, max_slots, sms, share);
+    case S_BITSET: return plan_group<PROB, S_BITSET, KeyT, CAND>(G, table, budget, max_slots, sms, share);
+    case S_BB: return plan_group<PROB, S_BB, KeyT, CAND>(G, table, budget, max_slots, sms, share);
+    default: return plan_group<PROB, S_BITSET_BB, KeyT, CAND>(G, table, budget, max_slots, sms, share);
   }
 }
 template <int PROB, class KeyT>
-ts_status plan_group_cand(Group& G, std::vector<BatchJobDev>& table, int64_t budget, int32_t max_slots, int sms) {
-  return G.cand ? plan_group_st<PROB, KeyT, true>(G, table, budget, max_slots, sms)
-                : plan_group_st<PROB, KeyT, false>(G, table, budget, max_slots, sms);
+ts_status plan_group_cand(Group& G, std::vector<BatchJobDev>& table, int64_t budget, int32_t max_slots, int sms,
+                          const DevBuf* share) {
+  return G.cand ? plan_group_st<PROB, KeyT, true>(G, table, budget, max_slots, sms, share)
+                : plan_group_st<PROB, KeyT, false>(G, table, budget, max_slots, sms, share);
+}
+ts_status plan_any(Group& G, std::vector<BatchJobDev>& table, int64_t budget, int32_t max_slots, int sms,
+                   const DevBuf* share) {
+  if (G.problem == P_MDP)
+    return G.wide ? plan_group_cand<P_MDP, long long>(G, table, budget, max_slots, sms, share)
+                  : plan_group_cand<P_MDP, int32_t>(G, table, budget, max_slots, sms, share);
+  return G.wide ? plan_group_cand<P_MAXBS, long long>(G, table, budget, max_slots, sms, share)
+                : plan_group_cand<P_MAXBS, int32_t>(G, table, budget, max_slots, sms, share);
 }
 
 // CTAs per solve that sweeps (pinned, or without the candidate pass) when the
@@ -460,6 +487,7 @@ ts_status ts_batch_create(const ts_batch_job* jobs, int32_t count, const ts_batc
     H.kind = J.graph->kind;
     H.num_pert = std::max(1, std::min(p.gamma, H.n) / 2);  // GPU-MAXBS-CSR.cu:433-434
     H.cluster = J.cluster;
+    H.open = J.cluster == 0;
     H.work = (double)H.m * (H.n - H.m) * (double)std::max<int64_t>(1, p.max_iter);
   }
   const int32_t device = jobs[0].graph->device;
@@ -546,6 +574,30 @@ ts_status ts_batch_create(const ts_batch_job* jobs, int32_t count, const ts_batc
     G.job_off = off;
     off += (long long)G.jobs.size();
   }
+  // Graphs of equal weights: ties may leave most iterations of a solve to the
+  // sweeps, on as few CTAs as suit the candidate pass (unit cliques, complete
+  // bipartite graphs: 5 to 7 times the time of the sweeps' own clusters).
+  // Such a solve is given up early and run by a launch of the sweeps' kernel
+  // behind the group's.
+  long long left_words = 0;
+  for (auto& G : b->groups) {
+    int32_t cs = 0;
+    for (const HostJob* H : G.jobs)
+      if (G.cand && equal_weights(H->g)) cs = std::max(cs, H->open ? auto_cluster(H->work, total, sms) : G.cluster);
+    if (!cs) continue;
+    G.swept.reset(new Group);
+    Group& S = *G.swept;
+    S.problem = G.problem;
+    S.kind = G.kind;
+    S.wide = G.wide;
+    S.cluster = std::max(cs, G.cluster);
+    S.jobs = G.jobs;
+    S.work = G.work;
+    S.job_off = off;
+    off += (long long)S.jobs.size();
+    G.left_off = left_words;
+    left_words += (long long)S.jobs.size();
+  }
   long long sol_words = 0, init_words = 0, draw_words = 0;
   std::vector<long long> sol_off(count), init_at(count), draw_at(count);
   for (int32_t q = 0; q < count; q++) {
@@ -562,16 +614,17 @@ ts_status ts_batch_create(const ts_batch_job* jobs, int32_t count, const ts_batc
   if ((rc = b->best.alloc(4 * (size_t)std::max<long long>(1, sol_words), "alloc batch best solutions")) != TS_OK)
     return rc;
   if ((rc = b->results.alloc(sizeof(BatchResultDev) * (size_t)count, "alloc batch results")) != TS_OK) return rc;
-  if ((rc = b->jobs.alloc(sizeof(BatchJobDev) * (size_t)count, "alloc batch jobs")) != TS_OK) return rc;
-  if ((rc = b->tickets.alloc(sizeof(unsigned int) * b->groups.size(), "alloc batch tickets")) != TS_OK) return rc;
+  if ((rc = b->jobs.alloc(sizeof(BatchJobDev) * (size_t)off, "alloc batch jobs")) != TS_OK) return rc;
+  if ((rc = b->tickets.alloc(4 * sizeof(unsigned int) * b->groups.size(), "alloc batch tickets")) != TS_OK) return rc;
+  if (left_words && (rc = b->left.alloc(4 * (size_t)left_words, "alloc batch lists")) != TS_OK) return rc;
   std::vector<int32_t> hi(std::max<long long>(1, init_words));
   std::vector<long long> hd(std::max<long long>(1, draw_words));
   for (int32_t q = 0; q < count; q++) {
     std::copy(hj[q].init.begin(), hj[q].init.end(), hi.begin() + init_at[q]);
     std::copy(hj[q].draws.begin(), hj[q].draws.end(), hd.begin() + draw_at[q]);
   }
-  std::vector<BatchJobDev> table(count);
-  for (auto& G : b->groups)
+  std::vector<BatchJobDev> table(off);
+  auto fill = [&](const Group& G, const Group* swept) {
     for (size_t q = 0; q < G.jobs.size(); q++) {
       const HostJob& H = *G.jobs[q];
       BatchJobDev& J = table[G.job_off + q];
@@ -591,7 +644,13 @@ ts_status ts_batch_create(const ts_batch_job* jobs, int32_t count, const ts_batc
       J.draws = b->draws.as<long long>() + draw_at[H.idx];
       J.draw_events = H.events;
       J.sol_off = sol_off[H.idx];
+      J.give_up = swept && equal_weights(H.g) ? swept->cluster / G.cluster : 0;
     }
+  };
+  for (const auto& G : b->groups) {
+    fill(G, G.swept.get());
+    if (G.swept) fill(*G.swept, nullptr);
+  }
   TS_CUDA(cudaMemcpyAsync(b->init.p, hi.data(), 4 * hi.size(), cudaMemcpyHostToDevice, b->stream));
   TS_CUDA(cudaMemcpyAsync(b->draws.p, hd.data(), 8 * hd.size(), cudaMemcpyHostToDevice, b->stream));
   // slot budget, shared out by work
@@ -603,13 +662,8 @@ ts_status ts_batch_create(const ts_batch_job* jobs, int32_t count, const ts_batc
   }
   for (auto& G : b->groups) {
     const int64_t gb = (int64_t)((double)budget * G.work / std::max(1.0, total));
-    if (G.problem == P_MDP)
-      rc = G.wide ? plan_group_cand<P_MDP, long long>(G, table, gb, o.max_slots, sms)
-                  : plan_group_cand<P_MDP, int32_t>(G, table, gb, o.max_slots, sms);
-    else
-      rc = G.wide ? plan_group_cand<P_MAXBS, long long>(G, table, gb, o.max_slots, sms)
-                  : plan_group_cand<P_MAXBS, int32_t>(G, table, gb, o.max_slots, sms);
-    if (rc != TS_OK) return rc;
+    if ((rc = plan_any(G, table, gb, o.max_slots, sms, nullptr)) != TS_OK) return rc;
+    if (G.swept && (rc = plan_any(*G.swept, table, gb, o.max_slots, sms, G.pool.get())) != TS_OK) return rc;
     b->info.slots += G.slots;
     b->info.slot_bytes += (int64_t)G.pool->bytes;
   }
@@ -633,12 +687,18 @@ ts_status ts_batch_create(const ts_batch_job* jobs, int32_t count, const ts_batc
   cudaError_t ce = cudaEventRecord(fork, b->stream);
   for (size_t gi = 0; gi < b->groups.size() && ce == cudaSuccess; gi++) {
     cudaStream_t s = b->gstreams[gi];
-    unsigned int* ticket = b->tickets.as<unsigned int>() + gi;
+    const Group& G = b->groups[gi];
+    // a ticket, another for the launch behind, the number of solves left to it
+    unsigned int* ticket = b->tickets.as<unsigned int>() + 4 * gi;
+    int32_t* left = G.swept ? b->left.as<int32_t>() + G.left_off : nullptr;
     ce = cudaStreamWaitEvent(s, fork, 0);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s);
-    if (ce == cudaSuccess)
-      ce = b->groups[gi].launch(s, b->jobs.as<BatchJobDev>(), b->results.as<BatchResultDev>(),
-                                b->best.as<int32_t>(), ticket);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(ticket, 0, 4 * sizeof(unsigned int), s);
+    auto launch = [&](const Group& X, unsigned int* next) {
+      return X.launch(s, b->jobs.as<BatchJobDev>(), b->results.as<BatchResultDev>(), b->best.as<int32_t>(), next, left,
+                      ticket + 2);
+    };
+    if (ce == cudaSuccess) ce = launch(G, ticket);
+    if (ce == cudaSuccess && left) ce = launch(*G.swept, ticket + 1);
     if (ce == cudaSuccess) ce = cudaEventRecord(b->events[gi + 1], s);
     if (ce == cudaSuccess) ce = cudaStreamWaitEvent(b->stream, b->events[gi + 1], 0);
   }
@@ -660,7 +720,7 @@ ts_status ts_batch_create(const ts_batch_job* jobs, int32_t count, const ts_batc
   b->info.jobs = count;
   b->info.groups = (int32_t)b->groups.size();
   b->info.input_bytes = (int64_t)(b->init.bytes + b->draws.bytes + b->best.bytes + b->results.bytes +
-                                  b->jobs.bytes + b->tickets.bytes);
+                                  b->jobs.bytes + b->tickets.bytes + b->left.bytes);
   b->info.best_sol_words = sol_words;
   *out = b.release();
   return TS_OK;

@@ -134,13 +134,22 @@ CandPlan cand_slices(const ts_graph* g, int32_t problem, int32_t m, bool wide, i
   return p;
 }
 
+bool equal_weights(const ts_graph* g) {
+  if (g->max_degree < 0) {
+    int64_t d = 0;
+    for (int32_t v = 0; v < g->n; v++) d = std::max(d, g->h_rowptr[v + 1] - g->h_rowptr[v]);
+    g->max_degree = d;
+  }
+  return !g->neg_w && g->max_wdeg == g->max_degree * g->max_abs_w;
+}
+
 // In a complete graph of equal weights all vertices of a side are alike: every
 // pair ties and the pass never settles an iteration.  Its shared memory would
 // only keep other CTAs of the sweeps off the SM (200 MDP solves of n = 600: 92
 // ms without it, 175 with it).  With both signs (weights of 1 and -1) the
 // contributions differ.
 static bool every_pair_ties(const ts_graph* g) {
-  return !g->neg_w && g->entries == (int64_t)g->n * (g->n - 1) && g->max_wdeg == (g->n - 1) * g->max_abs_w;
+  return g->entries == (int64_t)g->n * (g->n - 1) && equal_weights(g);
 }
 
 CandPlan cand_persist(const ts_graph* g, int32_t problem, int32_t m, bool wide, int32_t pass, int cs) {

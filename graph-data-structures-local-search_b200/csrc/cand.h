@@ -25,6 +25,9 @@ CandPlan cand_slices(const ts_graph* g, int32_t problem, int32_t m, bool wide, i
 // not apply: a pinned sweep, a graph on which every pair ties, or a state too
 // large for the cluster.
 CandPlan cand_persist(const ts_graph* g, int32_t problem, int32_t m, bool wide, int32_t pass, int cs);
+// Whether the graph's weights may all be equal and positive: its heaviest row
+// says so (a row of weights that happen to be the largest does too).
+bool equal_weights(const ts_graph* g);
 // Cluster size of a persistent solve whose caller leaves it open; 0 when no
 // cluster has the pass.
 int cand_cluster(const ts_graph* g, int32_t problem, int32_t m, bool wide, int32_t pass);

@@ -6,14 +6,13 @@
 
 #include "cand.cuh"
 #include "sweep.cuh"
-#include "topup.h"
 
 namespace tsb {
 
 struct BatchResultDev {
   long long iterations, evaluations, cur, best, best_true, perturbations;
   int32_t stopped, err;
-  int32_t complete, pad;  // complete: written when the solve has ended (served: until then iterations alone)
+  int32_t complete, given_up;  // complete: written when the solve has ended (served: until then iterations alone)
 };
 
 __device__ __forceinline__ long long block_sum(long long v, long long* sc) {
@@ -190,6 +189,9 @@ __device__ void slot_finish(const DevGraph& g, const DevSolver<KeyT>& s, BatchRe
   __syncthreads();
 }
 
+constexpr int32_t kTryFails = 4;   // tries of the candidate pass in a row that settle nothing
+constexpr int32_t kTrySweeps = 8;  // and the sweeps between two more of them, at most
+
 // Shared memory of the candidate pass in kernels that have it.
 template <bool CAND, class KeyT>
 struct CandSharedIf {
@@ -202,10 +204,13 @@ struct CandSharedIf<false, KeyT> {};
 // cluster: the candidate pass where the solve has it, else (and for the
 // iterations it leaves) round-robin tiles, the leader merging the records over
 // distributed shared memory and applying the move.  A try of the candidate pass
-// that stops again at once moves the whole state to shared memory and back, so
-// stops in quick succession double the sweeps between tries (bisection of n =
-// 150 with ties everywhere, 2,000 iterations: 149 ms with a try at each, 120.5
-// with fewer, 119 with the sweep pinned).  Every CTA of the cluster calls it.
+// that stops at once moves the whole state to shared memory and back: once four
+// in a row settled nothing, up to eight sweeps come between two of them
+// (bisection of n = 150 with ties everywhere, 2,000 iterations: 149 ms with a try
+// at each, 121 with fewer, 119 with the sweep pinned).  Not sooner: a sweep on few
+// CTAs takes many times the pass's iteration, and ties that pass are common in
+// graphs of equal weights.
+// Every CTA of the cluster calls it.
 //
 // CAND: the solve has the candidate pass.  Kernels for solves without it
 // (pinned sweeps above all) are compiled without it: its registers and its code
@@ -213,20 +218,30 @@ struct CandSharedIf<false, KeyT> {};
 // the tile pass 23.5 -> 38.6 ms, 300 bisections 112 -> 140, on the per-row pass
 // 302 -> 387).
 //
+// give_up > 0: a kernel without the pass can sweep the solve, on that many times
+// the CTAs.  It returns false once eight iterations were swept and their share
+// says that this is the better way.  Iterations without an allowed pair do not
+// count: the pass saves a sweep there.  A served solve goes on from its state;
+// a batched one starts again, so that the rest must be worth all of it.
+//
 // TIMED (served): sweeps end after `budget_ns` too, wherever the search is then.
 // How many iterations of a solve the candidate pass will leave to them is not
 // known beforehand, and other requests wait for the launch.
 template <int PROB, int ST, class KeyT, bool CAND, bool TIMED>
-__device__ void cluster_iterate(const DevGraph& g, const DevSolver<KeyT>& s, long long stop_at,
-                                [[maybe_unused]] long long budget_ns, cooperative_groups::cluster_group& cl,
-                                TailShared& sh, CtaRec& s_rec, CandSharedIf<CAND, KeyT>& s_cand) {
+__device__ bool cluster_iterate(const DevGraph& g, const DevSolver<KeyT>& s, long long stop_at,
+                                [[maybe_unused]] long long budget_ns, [[maybe_unused]] int32_t give_up,
+                                cooperative_groups::cluster_group& cl, TailShared& sh, CtaRec& s_rec,
+                                CandSharedIf<CAND, KeyT>& s_cand) {
   [[maybe_unused]] extern __shared__ __align__(16) unsigned char smem_raw[];
   const unsigned rank = cl.block_rank(), cs = cl.num_blocks();
   const int tid = threadIdx.x;
   const int ntiles = s.n_row_blocks * s.n_chunks;
   const DevState* st = s.st;
-  long long last = CAND ? __ldcg(&st->iter) : 0;  // at the last try of the candidate pass
-  int32_t sweeps = 1, wait = 0;                   // between tries; left until the next
+  const long long first = CAND ? __ldcg(&st->iter) : 0;
+  long long at = first;                     // the iteration before the last sweep
+  bool moving = false;                      // it was one that moves, if it finds a pair
+  int32_t fails = 0, wait = 0, swept = 0;   // tries in a row that settled nothing; sweeps until the next; swept iterations
+  bool finished = true;
   [[maybe_unused]] __shared__ int32_t late;       // the leader's word on the time
   [[maybe_unused]] const long long began = TIMED ? (long long)global_ns() : 0;
   for (;;) {
@@ -237,13 +252,27 @@ __device__ void cluster_iterate(const DevGraph& g, const DevSolver<KeyT>& s, lon
     const long long it = __ldcg(&st->iter);
     if (__ldcg(&st->done) || it >= stop_at) break;
     const int mode = __ldcg(&st->mode);
-    if (tried) {
-      // (a try that found no allowed pair saved the sweep that would find it)
-      if (mode == 0) sweeps = (int32_t)sweeps_after(sweeps, it - last);
-      wait = mode == 0 ? sweeps : 1;
-      last = it;
+    if constexpr (CAND) {
+      if (moving && it > at) swept++;
+      if (tried) {
+        // (a try that found no allowed pair saved the sweep that would find it)
+        fails = mode != 0 || it > at + moving ? 0 : fails + 1;
+        wait = fails <= kTryFails ? 1 : min(1 << (fails - kTryFails), kTrySweeps);
+      }
+      if (give_up && swept >= 8) {
+        const float made = (float)(it - first), rest = (float)(stop_at - it), all = (float)(stop_at - first);
+        const float better = TIMED ? 2.f * swept - made
+                             : give_up > 1 ? 0.8f * rest * swept * give_up - all * made
+                                           : (2.f * swept >= made ? all - 32.f * made : 0.f);
+        if (better > 0.f) {
+          finished = false;
+          break;
+        }
+      }
+      wait--;
+      moving = mode == 0;
+      at = it;
     }
-    if (wait > 0) wait--;
     const long long D64 = __ldcg(&st->best) - __ldcg(&st->cur);
     long long k = LLONG_MIN, i = LLONG_MAX;
     for (int t = (int)rank; t < ntiles; t += (int)cs) {
@@ -269,6 +298,7 @@ __device__ void cluster_iterate(const DevGraph& g, const DevSolver<KeyT>& s, lon
     if (TIMED && *cl.map_shared_rank(&late, 0)) break;
   }
   if (TIMED) cl.sync();  // the leader stays until its word is read
+  return finished;
 }
 
 }  // namespace tsb

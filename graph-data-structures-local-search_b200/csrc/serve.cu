@@ -48,7 +48,7 @@ struct ServeJobDev {
   long long stop_at;       // this launch runs the solve up to this iteration
   long long budget_ns;     // and sweeps no longer than this
   int32_t need_init;
-  int32_t pad;
+  int32_t give_up;         // equal weights: leave a solve that is swept to the kernel without the pass
   BatchResultDev* out;     // written when the solve ends
   int32_t* best_out;
 };
@@ -71,14 +71,16 @@ serve_kernel(const ServeJobDev<KeyT>* __restrict__ jobs) {
     __threadfence();
   }
   cl.sync();
-  cluster_iterate<PROB, ST, KeyT, CAND, true>(J.g, J.s, J.stop_at < J.max_iter ? J.stop_at : J.max_iter, J.budget_ns, cl,
-                                              sh, s_rec, s_cand);
+  const bool finished = cluster_iterate<PROB, ST, KeyT, CAND, true>(
+      J.g, J.s, J.stop_at < J.max_iter ? J.stop_at : J.max_iter, J.budget_ns, J.give_up, cl, sh, s_rec, s_cand);
   if (rank == 0) {
     const DevState* st = J.s.st;
     if (__ldcg(&st->done) || __ldcg(&st->iter) >= J.max_iter)
       slot_finish<PROB, KeyT>(J.g, J.s, J.out, J.best_out, sc);
-    else if (threadIdx.x == 0)
+    else if (threadIdx.x == 0) {
       J.out->iterations = __ldcg(&st->iter);
+      J.out->given_up = !finished;
+    }
   }
 }
 
@@ -143,7 +145,7 @@ struct Req {
   bool plain = false, wide = false;
   bool cand = false;  // has the candidate pass (packed: on its cluster)
   int32_t cs = 1;
-  size_t smem = 16;  // packed: dynamic shared memory of one tile (tile_geometry)
+  size_t smem = 16, tile_smem = 16;  // packed: dynamic shared memory, and that of a tile alone
   // device resources
   ts_graph* g = nullptr;
   cudaStream_t stream = nullptr;   // plain: the graph's and solver's stream
@@ -265,6 +267,7 @@ ts_status build_packed(Req& r, int32_t kind) {
   s.cand_fav = cp.fav;
   s.cand_plus = cp.plus;
   s.cand_pairs = cp.pairs;
+  r.tile_smem = tg.smem;
   r.smem = std::max(tg.smem, cp.smem);
   s.P = (int64_t)m * delta;
   const int64_t entries = r.g->entries;
@@ -547,6 +550,7 @@ void ts_server::round() {
         J->stop_at = r.at + k;
         J->budget_ns = (long long)(1e9 * round_s);
         J->need_init = r.started ? 0 : 1;
+        J->give_up = r.cand && equal_weights(r.g) ? 1 : 0;
         J->out = r.d_res;
         J->best_out = r.d_best;
         smem = std::max(smem, r.smem);
@@ -629,6 +633,10 @@ void ts_server::round() {
       }
       if (!d.complete) {
         r.at = d.iterations;
+        if (d.given_up) {  // ties: the sweeps' kernel from here on
+          r.cand = false;
+          r.smem = r.tile_smem;
+        }
         continue;
       }
       ts_result res;

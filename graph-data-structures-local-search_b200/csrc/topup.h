@@ -3,19 +3,13 @@
 #pragma once
 #include <cstdint>
 
-#ifdef __CUDACC__
-#define TS_HOST_DEVICE __host__ __device__
-#else
-#define TS_HOST_DEVICE
-#endif
-
 namespace tsb {
 
 // Sweeps until the next try of the candidate pass, when the last try came after
 // `sweeps` of them and `gained` iterations have been made since: stops in
 // quick succession (ties everywhere) double them.
 constexpr int64_t kMaxSweeps = 4096;
-TS_HOST_DEVICE inline int64_t sweeps_after(int64_t sweeps, int64_t gained) {
+inline int64_t sweeps_after(int64_t sweeps, int64_t gained) {
   if (gained > 4 * sweeps) return 1;
   return 2 * sweeps < kMaxSweeps ? 2 * sweeps : kMaxSweeps;
 }

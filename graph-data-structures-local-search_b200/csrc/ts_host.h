@@ -188,6 +188,7 @@ struct ts_graph {
   int64_t device_bytes() const {
     return (int64_t)(rowptr.bytes + adj.bytes + bits.bytes + hoff.bytes + hkey.bytes + hval.bytes + rev.bytes + wrange.bytes);
   }
+  mutable int64_t max_degree = -1;  // computed on first use
   mutable int64_t deg90 = -1;  // 90th-percentile degree, computed on first use
 };
 

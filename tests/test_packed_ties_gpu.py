@@ -149,3 +149,63 @@ def test_only_equal_weights_tie_everywhere(gpu, weights, groups):
         assert (r.iterations, r.cur, r.best, r.best_true) == (o.iterations, o.cur, o.best, o.best_true)
     b.close()
     g.close()
+
+
+def tied(family, n):
+    if family == "bipartite":
+        u, v = (x.ravel() for x in np.meshgrid(np.arange(n // 2), np.arange(n // 2, n)))
+    else:  # cliques of 20
+        a, b = np.triu_indices(20, 1)
+        first = np.arange(n // 20)[:, None] * 20
+        u, v = (first + a).ravel(), (first + b).ravel()
+    return u.astype(np.int32), v.astype(np.int32), np.ones(len(u), np.int32)
+
+
+@pytest.mark.parametrize("family", ["bipartite", "cliques"])
+@pytest.mark.parametrize("problem", [T.PROBLEM_MDP, T.PROBLEM_MAXBS])
+def test_solves_given_up_by_the_candidate_pass(gpu, problem, family):
+    """Equal weights that tie for good: the solves are run again by the sweeps'
+    kernel on its own clusters, beside others of their group that are not; twice,
+    as a replay clears the list; with the sweep's clusters and explicit ones."""
+    n, drop = 400, problem == T.PROBLEM_MDP
+    kw = dict(m=40 if drop else 0, max_iter=200, tenure_policy=FIXED, tenure=8, piter=60, gamma=16)
+    edges = [tied(family, n), sparse(n, 8, 3)]
+    graphs = [T.Graph(n, *e, "csr", drop_self_loops=drop) for e in edges]
+    want = [[O.run(O.Graph(n, *e, drop_self_loops=drop), O.MDP if drop else O.MAXBS, threads=0, seed=k + 1, **kw)
+             for k in range(3)] for e in edges]
+    specs = [(T.BatchJobSpec(g, problem, seed=k + 1, cluster=cs, **kw), w[k])
+             for cs in (0, 1, 4) for g, w in zip(graphs, want) for k in range(3)]
+    b = T.Batch([s for s, _ in specs])
+    for _ in range(2):
+        for r, (_, o) in zip(b.run(), specs):
+            assert (r.iterations, r.evaluations, r.cur, r.best, r.best_true, r.stopped, r.device_error) == \
+                   (o.iterations, o.evaluations, o.cur, o.best, o.best_true, o.stopped, 0)
+    b.close()
+    for g in graphs:
+        g.close()
+
+
+def test_given_up_solves_get_the_sweeps_clusters(gpu):
+    """Eight bisections of 2,000 vertices in unit cliques: 7 times the sweeps' time
+    on the candidate pass's one CTA each."""
+    n = 2000
+    g = T.Graph(n, *tied("cliques", n), "csr", drop_self_loops=False)
+
+    def batch_time(sweep):
+        b = T.Batch([T.BatchJobSpec(g, T.PROBLEM_MAXBS, max_iter=150, tenure_policy=FIXED, tenure=20, piter=100, seed=k + 1,
+                                    sweep=sweep) for k in range(8)])
+        best = 1e9
+        for _ in range(4):
+            t = time.perf_counter()
+            b.launch()
+            b.sync()
+            best = min(best, time.perf_counter() - t)
+        out = [(r.cur, r.best, r.iterations) for r in b.results()]
+        b.close()
+        return best, out
+
+    pinned, want = min((batch_time(s) for s in (T.PASS_TILE, T.PASS_ROWS)), key=lambda x: x[0])
+    auto, got = batch_time(T.PASS_AUTO)
+    g.close()
+    assert got == want
+    assert auto < 3 * pinned, (auto, pinned)

@@ -100,3 +100,20 @@ def test_plain_solves_go_on_after_a_hand_over(gpu):
     assert d.status == 0 and d.executor == "plain"
     assert (d.result.iterations, d.result.cur, d.result.best) == (r.iterations, r.cur, r.best)
     assert rounds <= 150, rounds
+
+
+@pytest.mark.parametrize("problem", [T.PROBLEM_MDP, T.PROBLEM_MAXBS])
+def test_request_given_up_by_the_candidate_pass(gpu, problem):
+    """A packed request on a complete bipartite graph of equal weights goes on in
+    the sweeps' kernel, from the state it had."""
+    n = 500
+    u, v = (x.ravel().astype(np.int32) for x in np.meshgrid(np.arange(n // 2), np.arange(n // 2, n)))
+    q = dict(m=50 if problem == T.PROBLEM_MDP else 0, max_iter=600, tenure_policy=FIXED, tenure=9, seed=2, piter=150, gamma=20)
+    req = (n, u, v, np.ones(len(u), np.int32), problem, "hash", q)
+    other = (400, *er(400, 9, 5), problem, "hash", dict(q, m=min(q["m"], 40)))
+    for d, (rn, ru, rv, rw, p, kind, kw) in zip(serve([req, other], round_ms=2.0)[0], (req, other)):
+        r = alone(rn, ru, rv, rw, p, kind, **kw)
+        assert d.status == 0 and d.executor == "packed"
+        assert (d.result.iterations, d.result.cur, d.result.best, d.result.best_true, d.result.stopped) == \
+               (r.iterations, r.cur, r.best, r.best_true, r.stopped)
+        np.testing.assert_array_equal(d.result.best_sol, r.best_sol)
